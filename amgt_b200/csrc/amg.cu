@@ -636,6 +636,9 @@ void free_level(Level &v, cudaStream_t s)
     amgt_pbsr_free(&v.pAs, (amgt_stream_t)s);
     amgt_pbsr_free(&v.pP, (amgt_stream_t)s);
     amgt_pbsr_free(&v.pR, (amgt_stream_t)s);
+    sell_free(v.sA, s);
+    sell_free(v.sP, s);
+    sell_free(v.sR, s);
     free_ptr(v.inv_l1, s);
     free_ptr(v.f, s);
     free_ptr(v.u, s);
@@ -803,14 +806,18 @@ int cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s)
             AMGT_TRY(pbsr_residual(&v.pA, f, v.u, v.t, s, h->sm_count));
             AMGT_TRY(pbsr_spmv(&v.pR, 1.0, v.t, 0.0, lv[l + 1].f, s, h->sm_count));
         } else {
-            AMGT_TRY(spmv_residual(l == 0 ? h->resid_prec0 : v.prec, &v.A, f, v.u, v.t, s, h->sm_count));
+            AMGT_TRY(op_residual(l == 0 ? h->resid_prec0 : v.prec, &v.A, v.sA, f, v.u, v.t, s, h->sm_count));
             Level &nx = lv[l + 1];
             if (l + 1 < L - 1 && restrict_fusable(&v.R)) {  // the next level smooths: fuse its first sweep
-                AMGT_TRY(spmv_restrict_jacobi0(v.prec_transfer, &v.R, v.t, nx.f, nx.inv_l1, w, nx.u, s,
-                                               h->sm_count));
+                const int mode = storage_mode(&v.R, v.prec_transfer);
+                if (sell_has(v.sR, mode))
+                    AMGT_TRY(sell_restrict_jacobi0(v.sR, mode, v.t, nx.f, nx.inv_l1, w, nx.u, s, h->sm_count));
+                else
+                    AMGT_TRY(spmv_restrict_jacobi0(v.prec_transfer, &v.R, v.t, nx.f, nx.inv_l1, w, nx.u, s,
+                                                   h->sm_count));
                 have_u = true;
             } else {
-                AMGT_TRY(amgt_spmv(v.prec_transfer, 1.0, &v.R, v.t, 0.0, nx.f, (amgt_stream_t)s));
+                AMGT_TRY(op_spmv(v.prec_transfer, 1.0, &v.R, v.sR, v.t, 0.0, nx.f, s, h->sm_count));
             }
         }
     }
@@ -827,9 +834,12 @@ int cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s)
             AMGT_TRY(pbsr_spmv(&v.pP, 1.0, lv[l + 1].s, 1.0, v.u, s, h->sm_count));
             AMGT_TRY(pbsr_jacobi(l == 0 ? &v.pAs : &v.pA, v.inv_l1, w, f, v.u, out, s, h->sm_count));
         } else {
-            AMGT_TRY(amgt_spmv(v.prec_transfer, 1.0, &v.P, lv[l + 1].s, 1.0, v.u, (amgt_stream_t)s));
-            AMGT_TRY(spmv_jacobi(l == 0 ? h->prm.smooth_prec0 : v.prec, &v.A, v.inv_l1, w, f, v.u, out, s,
-                                 h->sm_count));
+            AMGT_TRY(op_spmv(v.prec_transfer, 1.0, &v.P, v.sP, lv[l + 1].s, 1.0, v.u, s, h->sm_count));
+            const int prec = l == 0 ? h->prm.smooth_prec0 : v.prec, mode = storage_mode(&v.A, prec);
+            if (sell_has(v.sA, mode))
+                AMGT_TRY(sell_jacobi(v.sA, mode, v.inv_l1, w, f, v.u, out, s, h->sm_count));
+            else
+                AMGT_TRY(spmv_jacobi(prec, &v.A, v.inv_l1, w, f, v.u, out, s, h->sm_count));
         }
     }
     return AMGT_OK;
@@ -847,6 +857,8 @@ int pcg_iteration(amgt_amg *h, double *x, cudaStream_t s)
 {
     Level &v0 = h->lv[0];
     if (h->prm.packed) AMGT_TRY(pbsr_dot(&v0.pA, h->p, h->q, h->part, h->grid0, s));
+    else if (const int mode = storage_mode(&v0.A, AMGT_DOUBLE); sell_has(v0.sA, mode))
+        AMGT_TRY(sell_dot(v0.sA, mode, h->p, h->q, h->part, s, h->sm_count));
     else AMGT_TRY(spmv_dot(AMGT_DOUBLE, &v0.A, h->p, h->q, h->part, h->grid0, s));
     AMGT_LAUNCH_PDL(reduce_kernel, 1, kDotThreads, 0, s, h->part, h->grid0, h->scal, (int)S_PQ, (int)OP_ALPHA);
     AMGT_LAUNCH_PDL(axpy2_dot_kernel, kDotGrid, kDotThreads, 0, s, h->n0, h->scal, h->p, h->q, x, h->r, h->part);
@@ -967,7 +979,7 @@ int gm_iteration(amgt_amg *h, cudaStream_t s, int use_cond, cudaGraphConditional
     AMGT_TRY(cycle(h, h->gm_vin, h->gm_zout, s));
     AMGT_LAUNCH_PDL(gm_store_z_kernel, grid_n(h, n), 256, 0, s, n, (const double *)h->gm_zout, (const int *)h->gm_j,
                     h->gmZ);
-    AMGT_TRY(amgt_spmv(h->prm.inner_prec0, 1.0, &h->lv[0].A, h->gm_zout, 0.0, h->gm_w, (amgt_stream_t)s));
+    AMGT_TRY(op_spmv(h->prm.inner_prec0, 1.0, &h->lv[0].A, h->lv[0].sA, h->gm_zout, 0.0, h->gm_w, s, h->sm_count));
     AMGT_LAUNCH_PDL(gm_mdot_kernel, kDotGrid, kDotThreads, 0, s, n, (const float *)h->gmV, (const int *)h->gm_j,
                     (const double *)h->gm_w, h->gm_part);
     AMGT_LAUNCH_PDL(gm_mdot_reduce_kernel, 1, 1024, 0, s, (const double *)h->gm_part, kDotGrid, (const int *)h->gm_j,
@@ -1039,7 +1051,7 @@ int fgmres_ir_solve(amgt_amg *h, const double *b, double *x, int *iterations, do
     bool graph_ran = false;
     for (int outer = 0; outer < h->prm.max_outer + 1; ++outer) {
         // fp64 residual of the current x (the refinement's residual)
-        AMGT_TRY(spmv_residual(AMGT_DOUBLE, &v0.A, b, x, h->r, s, h->sm_count));
+        AMGT_TRY(op_residual(AMGT_DOUBLE, &v0.A, v0.sA, b, x, h->r, s, h->sm_count));
         AMGT_TRY(dot(h, h->r, h->r, S_RR, OP_STORE, s));
         AMGT_CUDA_TRY(cudaMemcpyAsync(h->pinned, h->scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
         AMGT_CUDA_TRY(cudaMemcpyAsync(h->loop_pinned, h->loop_it, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1097,6 +1109,22 @@ int fgmres_ir_solve(amgt_amg *h, const double *b, double *x, int *iterations, do
 }
 
 }  // namespace
+
+int amgt::op_spmv(int prec, double alpha, const amgt_bsr *A, const SellMat &S, const double *x, double beta,
+                  double *y, cudaStream_t s, int sm_count)
+{
+    const int mode = storage_mode(A, prec);
+    if (sell_has(S, mode)) return sell_spmv(S, mode, alpha, x, beta, y, s, sm_count);
+    return amgt_spmv(prec, alpha, A, x, beta, y, (amgt_stream_t)s);
+}
+
+int amgt::op_residual(int prec, const amgt_bsr *A, const SellMat &S, const double *f, const double *u, double *r,
+                      cudaStream_t s, int sm_count)
+{
+    const int mode = storage_mode(A, prec);
+    if (sell_has(S, mode)) return sell_residual(S, mode, f, u, r, s, sm_count);
+    return spmv_residual(prec, A, f, u, r, s, sm_count);
+}
 
 int amgt::amg_cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s) { return cycle(h, rhs0, out0, s); }
 
@@ -1187,9 +1215,12 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
     int64_t *xflags = nullptr;
     std::vector<char> fused16(3 * (size_t)(num_interp + 1), 0);
     bool l1_fused0 = false;  // level 0's l1 norms written by A's conversion
+    std::vector<SellJob> sell;         // operators that get a sliced copy, ...
+    std::vector<int64_t> sell_meas;    // ... and its size as measured on the device
+    const size_t nflags = fused16.size(), nslots = 3 * nflags;  // exactness flags, then two slots per sliced copy
     pm.mark(-1, s);
-    if ((rc = alloc_n(&xflags, fused16.size(), s))) goto fail;
-    if (cudaMemsetAsync(xflags, 0, sizeof(int64_t) * fused16.size(), s) != cudaSuccess) {
+    if ((rc = alloc_n(&xflags, nslots, s))) goto fail;
+    if (cudaMemsetAsync(xflags, 0, sizeof(int64_t) * nslots, s) != cudaSuccess) {
         rc = AMGT_ERR_CUDA;
         goto fail;
     }
@@ -1403,6 +1434,17 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
         }
         free_ptr(dense, s);
     }
+    // sizes of the larger operators' sliced copies, read back with the
+    // exactness bits
+    if (!h->prm.packed) {
+        for (int l = 0; l < L; ++l) {
+            Level &v = h->lv[l];
+            if (l < L - 1 && sell_wanted(&v.A)) sell.push_back({&v.A, 0u, &v.sA});
+            if (l < L - 1 && sell_wanted(&v.P)) sell.push_back({&v.P, 0u, &v.sP});
+            if (l < L - 1 && sell_wanted(&v.R)) sell.push_back({&v.R, 0u, &v.sR});
+        }
+        if ((rc = sell_measure(sell, xflags + nflags, s, h->sm_count))) goto fail;
+    }
     // exact narrow storage of the operators used in fp64 (level 0, fp64
     // levels and transfers): one value check each, one read-back per 15
     if (h->prm.exact_storage) {
@@ -1428,19 +1470,26 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
             rc = bsr_exact_check(mats[i].first, xflags + slot, &o, s, h->sm_count);
             own16[slot] = o;
         }
-        std::vector<int64_t> f(fused16.size(), 0);
+        std::vector<int64_t> f(nflags + 2 * sell.size(), 0);
         for (size_t i0 = 0; i0 < f.size() && !rc; i0 += 63) {
             const int k = (int)std::min<size_t>(63, f.size() - i0);
             const int64_t *hf = nullptr;
             if ((rc = read_back(xflags + i0, k, s, &hf))) break;
             for (int i = 0; i < k; ++i) f[i0 + i] = hf[i];  // the pinned slots are reused by later calls
         }
+        sell_meas.assign(f.begin() + nflags, f.end());
         for (size_t i = 0; i < mats.size() && !rc; ++i) {
             const int slot = mats[i].second;
             const int fs = (slot % 3 == 2 && fused16[slot]) ? slot - 1 : slot;  // R_l carried P_l's shadow
             rc = bsr_exact_apply(mats[i].first, f[fs], own16[slot] != 0, s);
         }
         if (rc) goto fail;
+    }
+    for (size_t i0 = sell_meas.size(); i0 < 2 * sell.size(); i0 = sell_meas.size()) {  // no flags were read back
+        const int k = (int)std::min<size_t>(63, 2 * sell.size() - i0);
+        const int64_t *hf = nullptr;
+        if ((rc = read_back(xflags + nflags + i0, k, s, &hf))) goto fail;
+        sell_meas.insert(sell_meas.end(), hf, hf + k);
     }
     // smoother data, shadows, work vectors
     for (int l = 0; l < L; ++l) {
@@ -1468,6 +1517,23 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
         if ((rc = alloc_n(&v.u, v.n, s)) || (rc = alloc_n(&v.t, v.n, s))) goto fail;
         if (l > 0 && ((rc = alloc_n(&v.f, v.n, s)) || (rc = alloc_n(&v.s, v.n, s)))) goto fail;
     }
+    // the sliced copies, in the storage types that the cycle's products read
+    for (SellJob &j : sell) {
+        for (int l = 0; l < L; ++l) {
+            const Level &v = h->lv[l];
+            auto use = [&](int prec) { j.storages |= 1u << sell_storage(storage_mode(j.A, prec)); };
+            if (j.A == &v.P || j.A == &v.R) use(v.prec_transfer);
+            if (j.A != &v.A) continue;
+            if (l > 0) {
+                use(v.prec);
+            } else {
+                use(h->resid_prec0);
+                use(h->prm.smooth_prec0);
+                use(fgm ? h->prm.inner_prec0 : AMGT_DOUBLE);
+            }
+        }
+    }
+    if ((rc = sell_fill(sell, sell_meas.data(), s, h->sm_count))) goto fail;
     // coarsest: the inverse's singularity mark (one read-back)
     {
         const int64_t *hf = nullptr;
@@ -1480,7 +1546,10 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
     }
     // Krylov vectors and scalars
     h->n0 = h->lv[0].n;
-    h->grid0 = h->prm.packed ? pbsr_grid(&h->lv[0].pA, h->sm_count) : epi_grid(&h->lv[0].A, h->sm_count);
+    h->grid0 = h->prm.packed ? pbsr_grid(&h->lv[0].pA, h->sm_count)
+               : sell_has(h->lv[0].sA, storage_mode(&h->lv[0].A, AMGT_DOUBLE))
+                   ? sell_dot_grid(h->lv[0].sA, h->sm_count)
+                   : epi_grid(&h->lv[0].A, h->sm_count);
     if ((rc = alloc_n(&h->r, h->n0, s)) || (rc = alloc_n(&h->z, h->n0, s)) || (rc = alloc_n(&h->p, h->n0, s)) ||
         (rc = alloc_n(&h->q, h->n0, s)) || (rc = alloc_n(&h->scal, S_NSCAL, s)) ||
         (rc = alloc_n(&h->part, std::max(h->grid0, kDotGrid), s)) || (rc = alloc_n(&h->loop_it, 1, s)) ||
@@ -1546,7 +1615,7 @@ int amgt_amg_solve(amgt_amg *h, const double *b, double *x, int *iterations, dou
     Level &v0 = h->lv[0];
     h->hist.clear();
     // r = b - A x, ||b||^2, ||r||^2
-    AMGT_TRY(spmv_residual(AMGT_DOUBLE, &v0.A, b, x, h->r, s, h->sm_count));
+    AMGT_TRY(op_residual(AMGT_DOUBLE, &v0.A, v0.sA, b, x, h->r, s, h->sm_count));
     AMGT_TRY(dot(h, b, b, S_BB, OP_STORE, s));
     AMGT_TRY(dot(h, h->r, h->r, S_RR, OP_STORE, s));
     AMGT_CUDA_TRY(cudaMemcpyAsync(h->pinned, h->scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));

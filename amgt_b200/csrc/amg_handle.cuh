@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "amgt_internal.cuh"
+#include "sell.cuh"
 
 namespace amgt {
 
@@ -20,6 +21,7 @@ void free_batch(Batch *b, cudaStream_t s);
 struct Level {
     amgt_bsr A{}, P{}, R{};
     amgt_pbsr pA{}, pAs{}, pP{}, pR{};  // packed: cycle operator, level-0 smoother, transfers
+    SellMat sA, sP, sR;                 // sliced copies of the larger operators (sell.cu)
     double *inv_l1 = nullptr;
     double *f = nullptr, *u = nullptr, *t = nullptr, *s = nullptr;
     int n = 0;
@@ -73,6 +75,12 @@ struct amgt_amg {
 };
 
 namespace amgt {
+// The cycle's products: on the sliced copy S of A when it holds the values
+// that `prec` reads, else on the blocks (amg.cu).
+int op_spmv(int prec, double alpha, const amgt_bsr *A, const SellMat &S, const double *x, double beta, double *y,
+            cudaStream_t s, int sm_count);
+int op_residual(int prec, const amgt_bsr *A, const SellMat &S, const double *f, const double *u, double *r,
+                cudaStream_t s, int sm_count);
 // z = M r: one V(1,1) cycle of h's hierarchy (amg.cu)
 int amg_cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s);
 // amgt_amg_setup with the coarsest operator inverted per diagonal block:

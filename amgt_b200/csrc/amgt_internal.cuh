@@ -127,6 +127,10 @@ void tune_forget(const amgt_bsr *A);
 // y = beta * y (y = 0 when beta == 0) over n entries (spmv.cu).
 int scale_vector(long long n, double beta, double *y, int sm_count, cudaStream_t s);
 
+// Value mode that products of A at `prec` read (an AMGT_* precision or an
+// exact narrow storage mode of spmv_common.cuh).
+int storage_mode(const amgt_bsr *A, int prec);
+
 // Fused SpMV forms (spmv.cu): r = f - A u; u_out = u + w (f - A u) .* inv_l1;
 // out = A u with per-CTA partials of u . out (grid CTAs, from epi_grid);
 // l1 row norms (or their inverses).

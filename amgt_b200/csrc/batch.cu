@@ -221,7 +221,7 @@ int b_iteration(amgt_amg *h, Batch *b, double *x, cudaStream_t s, int use_cond, 
 {
     Level &v0 = h->lv[0];
     const int grid = std::min(b->ntiles, 8 * h->sm_count);
-    AMGT_TRY(amgt_spmv(AMGT_DOUBLE, 1.0, &v0.A, h->p, 0.0, h->q, (amgt_stream_t)s));
+    AMGT_TRY(op_spmv(AMGT_DOUBLE, 1.0, &v0.A, v0.sA, h->p, 0.0, h->q, s, h->sm_count));
     AMGT_TRY(dot_b(h, b, h->p, h->q, BS_PQ, BOP_ALPHA, s));
     AMGT_LAUNCH_PDL(b_axpy2_dot_kernel, grid, kBThreads, 0, s, b->ntiles, b->nsys, (const int *)b->tile_beg,
                     (const int *)b->tile_sys, (const double *)b->scal, (const double *)h->p, (const double *)h->q, x,
@@ -428,7 +428,7 @@ int amgt_amg_solve_batch(amgt_amg *h, const double *bvec, double *x, int *iterat
     const int ns = b->nsys;
     AMGT_CUDA_TRY(cudaMemsetAsync(b->cnt, 0, sizeof(int) * (ns + 2), s));
     AMGT_CUDA_TRY(cudaMemsetAsync(b->scal, 0, sizeof(double) * BS_NSLOT * ns, s));
-    AMGT_TRY(spmv_residual(AMGT_DOUBLE, &v0.A, bvec, x, h->r, s, h->sm_count));
+    AMGT_TRY(op_residual(AMGT_DOUBLE, &v0.A, v0.sA, bvec, x, h->r, s, h->sm_count));
     AMGT_TRY(dot_b(h, b, bvec, bvec, BS_BB, BOP_STORE, s));
     AMGT_TRY(dot_b(h, b, h->r, h->r, BS_RR, BOP_RR_TEST, s));
     AMGT_TRY(amg_cycle(h, h->r, h->z, s));
@@ -460,7 +460,7 @@ int amgt_amg_solve_batch(amgt_amg *h, const double *bvec, double *x, int *iterat
         }
     }
     // true residuals of the returned x, per system
-    AMGT_TRY(spmv_residual(AMGT_DOUBLE, &v0.A, bvec, x, h->r, s, h->sm_count));
+    AMGT_TRY(op_residual(AMGT_DOUBLE, &v0.A, v0.sA, bvec, x, h->r, s, h->sm_count));
     AMGT_TRY(dot_b(h, b, h->r, h->r, BS_RR, BOP_STORE, s));
     AMGT_CUDA_TRY(cudaMemcpyAsync(b->pinned, b->scal, sizeof(double) * 2 * ns, cudaMemcpyDeviceToHost, s));
     AMGT_CUDA_TRY(cudaMemcpyAsync(b->pinned + 2 * ns, b->cnt, sizeof(int) * (ns + 2), cudaMemcpyDeviceToHost, s));

@@ -355,7 +355,7 @@ static const void *value_array(const amgt_bsr *A, int prec)
 // fp32 inputs and the same fp32 sums at half the bytes), so that a reduced
 // precision never reads more value bytes than the fp64 form of the same
 // operator.  bf16 keeps its own rounding.
-static int storage_mode(const amgt_bsr *A, int prec)
+int storage_mode(const amgt_bsr *A, int prec)
 {
     if (prec == AMGT_FLOAT && A->exact_prec == AMGT_HALF && A->blcVal_fp16) return AMGT_HALF;
     if (prec != AMGT_DOUBLE) return prec;

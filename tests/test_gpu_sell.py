@@ -1,0 +1,78 @@
+"""GPU tests of the cycle's sliced operators (sell.cu), through the AMG solve
+that uses them: fp64 solves take the oracle's iterations with x within 1e-9
+of its (the bars of the block path, test_gpu_amg.py), on shapes that reach
+each form: 16-bit offsets, 32-bit columns (a slice's columns spread over more
+than 65,535), several lanes per row, ragged sizes, operators that get no copy
+because one long row would pad its slice, and reduced-precision storage."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(orc, kind):
+    if kind == "idx32":  # planes of 93,000 unknowns: a slice's columns span two of them
+        return orc.laplacian(310, 300, 3), orc.geometric_hierarchy(310, 300, 3)
+    if kind == "ragged":
+        return orc.laplacian(61, 53, 47), orc.geometric_hierarchy(61, 53, 47)
+    if kind == "lanes8":  # 24,360 rows of about 24 entries: eight lanes a row
+        return orc.varcoef27(30, 29, 28, seed=4), orc.geometric_hierarchy(30, 29, 28)
+    # "long_row": the first unknown coupled to every other one
+    import scipy.sparse as sp
+
+    dims = (48, 48, 24)
+    S = orc.laplacian(*dims).to_scipy().tolil()
+    n = S.shape[0]
+    S[0, 1:] = -1e-4
+    S[1:, 0] = -1e-4
+    S = sp.csr_matrix(S)
+    S = S + sp.diags(np.where(np.arange(n) == 0, 1e-4 * n, 1e-4))
+    S = sp.csr_matrix(S)
+    S.sort_indices()
+    return (orc.CSR(n, n, S.indptr.astype(np.int32), S.indices.astype(np.int32), S.data),
+            orc.geometric_hierarchy(*dims))
+
+
+def _solver(A, Ps, **kw):
+    from amgt_b200.amg import AmgSolver, default_params
+
+    return AmgSolver(to_dev(A), [to_dev(P) for P in Ps], default_params(**kw))
+
+
+@pytest.mark.parametrize("kind", ["idx32", "ragged", "lanes8", "long_row"])
+def test_fp64_solve_matches_the_oracle(amgt, orc, kind):
+    A, Ps = _problem(orc, kind)
+    b = A.to_scipy() @ orc.rand_uniform(3, A.n)
+    xo, it_o, _, _ = orc.Amg(A, Ps).solve(b)
+    amgt.set_level_policy([0])
+    try:
+        S = _solver(A, Ps)
+        x, it, rel = S.solve(torch.from_numpy(b).cuda())
+        S.free()
+    finally:
+        amgt.set_level_policy([])
+    assert it == it_o and rel <= 1e-8
+    assert np.linalg.norm(x.cpu().numpy() - xo) <= 1e-9 * np.linalg.norm(xo)
+
+
+@pytest.mark.parametrize("prec", [1, 2, 3])
+def test_reduced_levels_and_transfers_converge_fp64_verified(amgt, orc, prec):
+    """Level 0's smoother at fp32, the coarser levels and the transfers at
+    `prec` (fp32 / fp16 / bf16), on an operator no narrow storage holds
+    exactly: the fp64 residual reaches 1e-8."""
+    dims = (60, 58, 56)
+    A, Ps = orc.varcoef27(*dims, seed=5), orc.geometric_hierarchy(*dims)
+    b = A.to_scipy() @ orc.rand_uniform(4, A.n)
+    amgt.set_level_policy([0, prec])
+    try:
+        S = _solver(A, Ps, flexible=1, smooth_prec0=1)
+        x, it, rel = S.solve(torch.from_numpy(b).cuda())
+        S.free()
+    finally:
+        amgt.set_level_policy([])
+    r = b - A.to_scipy() @ x.cpu().numpy()
+    assert np.linalg.norm(r) <= 1.0000001e-8 * np.linalg.norm(b)
+    assert it < 60
