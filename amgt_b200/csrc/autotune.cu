@@ -119,8 +119,9 @@ int amgt_spmm_rm(int prec, int engine, double alpha, const amgt_bsr *A, int nvec
     cudaStream_t s = (cudaStream_t)stream;
     if (A->blc_num == 0 || A->col == 0) return scale_vector((long long)A->row * nvec, beta, Y, st->sm_count, s);
     if (!X || !A->blcPtr || !A->blcIdx) return AMGT_ERR_INVALID;
-    int kind = 1, wpc = 8;
-    if (engine == AMGT_ENGINE_CUDA_CORE) kind = 0;
+    // AUTO without a measured choice: the CUDA-core form, faster than the
+    // tensor-core one at every size measured (spmm_tc.cu)
+    int kind = engine == AMGT_ENGINE_TENSOR_CORE ? 1 : 0, wpc = 8;
     if (engine == AMGT_ENGINE_AUTO) {
         Choice c;
         if (lookup(A, prec, nvec, &c)) {

@@ -10,9 +10,10 @@
 //   correction          A D = R by PCG in lockstep over the columns (each
 //                       column its own alpha, beta, and its own stop at
 //                       inner_tol * ||R_v||), preconditioned by one V(1,1)
-//                       cycle; every operator through amgt_spmm_rm at its
-//                       level's precision (fp32 / fp16 / bf16 levels on the
-//                       tensor cores; level 0 at inner_prec0); X += D.
+//                       cycle; every operator one SpMM at its level's
+//                       precision (level 0 at inner_prec0) with the vector
+//                       passes around it fused into its epilogue
+//                       (spmm.cuh); X += D.
 // The correction's iteration loop is one CUDA graph launch (a conditional
 // while node whose body ends with the per-column convergence test).
 // Kernels use a lane per right-hand side and warps striding over rows, so
@@ -22,11 +23,9 @@
 #include <cstring>
 
 #include "amg_handle.cuh"
+#include "spmm.cuh"
 
 namespace amgt {
-
-int spmm_rowmajor(int prec, int kind, int wpc, const amgt_bsr *A, double alpha, const double *X, int nvec,
-                  double beta, double *Y, cudaStream_t s, int sm_count);
 
 // per-column scalars: scal[slot * 32 + v]
 enum { MS_BB = 0, MS_RR = 1, MS_RZ = 2, MS_PQ = 3, MS_ALPHA = 4, MS_BETA = 5, MS_RR0 = 6, MS_ACTIVE = 7,
@@ -101,16 +100,22 @@ __global__ void __launch_bounds__(kMvThreads) mv_dot_kernel(long long n, int nv,
     }
 }
 
-// sums the partials per column (warp v, fixed order) and applies op
+// sums the partials per column and applies op: warp w adds the CTAs w, w + 32,
+// ... of every column (a lane per column, coalesced), then the columns' 32
+// sums are added in warp order
 __global__ void __launch_bounds__(1024) mv_reduce_kernel(const double *__restrict__ part, int np, int nv,
                                                         double *__restrict__ scal, int slot, int op,
                                                         double inner_tol)
 {
     grid_dependency_wait();
+    __shared__ double sred[32][33];
+    double t = 0.0;
+    for (int k = threadIdx.x >> 5; k < np; k += 32) t += part[k * 32 + (threadIdx.x & 31)];
+    sred[threadIdx.x & 31][threadIdx.x >> 5] = t;
+    __syncthreads();
     const int v = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (v >= nv) return;
-    double t = 0.0;
-    for (int k = lane; k < np; k += 32) t += part[k * 32 + v];
+    t = sred[v][lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
     if (lane != 0) return;
@@ -175,29 +180,6 @@ __global__ void mv_xpby_kernel(long long n, int nv, const double *__restrict__ z
     }
 }
 
-// u = w f .* inv_l1 (smoothing from zero)
-__global__ void mv_jacobi_zero_kernel(long long n, int nv, const double *__restrict__ f,
-                                      const double *__restrict__ inv_l1, double w, double *__restrict__ u)
-{
-    grid_dependency_wait();
-    MV_LOOP(i, n)
-    {
-        if (live) u[i * nv + lane] = w * f[i * nv + lane] * inv_l1[i];
-    }
-}
-
-// out = u + w t .* inv_l1 (t = f - A u)
-__global__ void mv_jacobi_update_kernel(long long n, int nv, const double *__restrict__ u,
-                                        const double *__restrict__ t, const double *__restrict__ inv_l1, double w,
-                                        double *__restrict__ out)
-{
-    grid_dependency_wait();
-    MV_LOOP(i, n)
-    {
-        if (live) out[i * nv + lane] = u[i * nv + lane] + w * t[i * nv + lane] * inv_l1[i];
-    }
-}
-
 __global__ void mv_copy_kernel(long long count, const double *__restrict__ a, double *__restrict__ b)
 {
     grid_dependency_wait();
@@ -238,11 +220,14 @@ __global__ void mv_continue_kernel(cudaGraphConditionalHandle cond, int use_cond
                                    const double *__restrict__ scal, int *__restrict__ cnt, int max_iter,
                                    int *__restrict__ more_out)
 {
-    int any = 0;
-    for (int v = 0; v < nv; ++v) {
+    const int v = threadIdx.x;  // one warp, a lane per column
+    int active = 0;
+    if (v < nv) {
         if (scal[MS_ALPHA * 32 + v] != 0.0) ++cnt[v];  // the column took this iteration's step
-        any |= scal[MS_ACTIVE * 32 + v] != 0.0;        // and still needs one
+        active = scal[MS_ACTIVE * 32 + v] != 0.0;      // and still needs one
     }
+    const int any = __any_sync(FULL, active);
+    if (v != 0) return;
     const int k = ++cnt[32];
     const int more = (any && k < max_iter) ? 1 : 0;
     *more_out = more;
@@ -257,32 +242,31 @@ namespace {
 
 int mv_grid(long long n, int sm_count) { return grid_for(kMvThreads / 32, n, sm_count, 4); }
 
-// operator application through the SpMM (auto engine: autotuned or tensor cores)
-int apply(const amgt_amg *, int prec, const amgt_bsr *A, double alpha, const double *X, int nv, double beta,
-          double *Y, cudaStream_t s)
-{
-    return amgt_spmm_rm(prec, AMGT_ENGINE_AUTO, alpha, A, nv, X, beta, Y, (amgt_stream_t)s);
-}
-
 // Z = M R: one V(1,1) cycle on nv columns (the single-vector cycle of
-// amg.cu with every operator as an SpMM)
-int mv_cycle(amgt_amg *h, MultiRhs *mr, const double *rhs0, double *out0, cudaStream_t s)
+// amg.cu with every operator as an SpMM).  The sweep from a zero guess is
+// never stored: the residual and the correction form it from f entry by
+// entry, so that a level's cycle reads or writes 8 multivectors instead of
+// the 18 of separate sweeps, copies and updates.  dot: level 0's last sweep
+// also leaves the partials of rhs0 . out0 in mr->part (mv_apply_grid CTAs).
+int mv_cycle(amgt_amg *h, MultiRhs *mr, const double *rhs0, double *out0, bool dot, cudaStream_t s)
 {
     auto &lv = h->lv;
     const int L = (int)lv.size(), nv = mr->nv;
-    const double w = h->prm.relax_weight;
-    const int p0 = h->prm.inner_prec0;
+    MvArgs a{};
     for (int l = 0; l < L - 1; ++l) {
         Level &v = lv[l];
         MultiRhsLevel &m = mr->lv[l];
-        const double *f = (l == 0) ? rhs0 : m.f;
-        const int pl = l == 0 ? p0 : v.prec;
-        AMGT_LAUNCH_PDL(mv_jacobi_zero_kernel, mv_grid(v.n, h->sm_count), kMvThreads, 0, s, (long long)v.n, nv, f,
-                        (const double *)v.inv_l1, w, m.u);
-        AMGT_LAUNCH_PDL(mv_copy_kernel, grid_for(256, (long long)v.n * nv, h->sm_count, 8), 256, 0, s,
-                        (long long)v.n * nv, f, m.t);
-        AMGT_TRY(apply(h, pl, &v.A, -1.0, m.u, nv, 1.0, m.t, s));
-        AMGT_TRY(apply(h, v.prec_transfer, &v.R, 1.0, m.t, nv, 0.0, mr->lv[l + 1].f, s));
+        a = MvArgs{};
+        a.alpha = h->prm.relax_weight;
+        a.X = a.F = (l == 0) ? rhs0 : m.f;
+        a.inv_l1 = v.inv_l1;
+        a.Y = m.t;
+        AMGT_TRY(mv_apply(l == 0 ? h->prm.inner_prec0 : v.prec, MV_RESID0, &v.A, nv, a, s, h->sm_count));
+        a = MvArgs{};
+        a.alpha = 1.0;
+        a.X = m.t;
+        a.Y = mr->lv[l + 1].f;
+        AMGT_TRY(mv_apply(v.prec_transfer, MV_SPMM, &v.R, nv, a, s, h->sm_count));
     }
     Level &c = lv[L - 1];
     MultiRhsLevel &cm = mr->lv[L - 1];
@@ -294,25 +278,42 @@ int mv_cycle(amgt_amg *h, MultiRhs *mr, const double *rhs0, double *out0, cudaSt
     for (int l = L - 2; l >= 0; --l) {
         Level &v = lv[l];
         MultiRhsLevel &m = mr->lv[l];
-        const double *f = (l == 0) ? rhs0 : m.f;
-        double *out = (l == 0) ? out0 : m.s;
-        const int pl = l == 0 ? p0 : v.prec;
-        AMGT_TRY(apply(h, v.prec_transfer, &v.P, 1.0, mr->lv[l + 1].s, nv, 1.0, m.u, s));
-        AMGT_LAUNCH_PDL(mv_copy_kernel, grid_for(256, (long long)v.n * nv, h->sm_count, 8), 256, 0, s,
-                        (long long)v.n * nv, f, m.t);
-        AMGT_TRY(apply(h, pl, &v.A, -1.0, m.u, nv, 1.0, m.t, s));
-        AMGT_LAUNCH_PDL(mv_jacobi_update_kernel, mv_grid(v.n, h->sm_count), kMvThreads, 0, s, (long long)v.n, nv,
-                        (const double *)m.u, (const double *)m.t, (const double *)v.inv_l1, w, out);
+        a = MvArgs{};
+        a.alpha = h->prm.relax_weight;
+        a.X = mr->lv[l + 1].s;
+        a.F = (l == 0) ? rhs0 : m.f;
+        a.inv_l1 = v.inv_l1;
+        a.Y = m.u;
+        AMGT_TRY(mv_apply(v.prec_transfer, MV_CORRECT, &v.P, nv, a, s, h->sm_count));
+        a.X = m.u;
+        a.Y = (l == 0) ? out0 : m.s;
+        a.part = (dot && l == 0) ? mr->part : nullptr;
+        AMGT_TRY(mv_apply(l == 0 ? h->prm.inner_prec0 : v.prec, MV_JACOBI, &v.A, nv, a, s, h->sm_count));
     }
     return AMGT_OK;
 }
 
+// sums np partials per column and applies op
+int mv_reduce(amgt_amg *h, MultiRhs *mr, int np, int slot, int op, cudaStream_t s)
+{
+    AMGT_LAUNCH_PDL(mv_reduce_kernel, 1, 1024, 0, s, (const double *)mr->part, np, mr->nv, mr->scal, slot, op,
+                    h->prm.inner_tol);
+    return AMGT_OK;
+}
+
+// R . Z of the cycle just run (its own partials, or a dot when there is one level)
+int mv_cycle_dot(amgt_amg *h, MultiRhs *mr, const double *r, const double *z, int op, cudaStream_t s);
+
 int mv_dot(amgt_amg *h, MultiRhs *mr, const double *a, const double *b, int slot, int op, cudaStream_t s)
 {
     AMGT_LAUNCH_PDL(mv_dot_kernel, kMvGrid, kMvThreads, 0, s, h->n0, mr->nv, a, b, mr->part);
-    AMGT_LAUNCH_PDL(mv_reduce_kernel, 1, 1024, 0, s, (const double *)mr->part, kMvGrid, mr->nv, mr->scal, slot, op,
-                    h->prm.inner_tol);
-    return AMGT_OK;
+    return mv_reduce(h, mr, kMvGrid, slot, op, s);
+}
+
+int mv_cycle_dot(amgt_amg *h, MultiRhs *mr, const double *r, const double *z, int op, cudaStream_t s)
+{
+    if (h->lv.size() == 1) return mv_dot(h, mr, r, z, MS_RZ, op, s);
+    return mv_reduce(h, mr, mv_apply_grid(&h->lv[0].A, mr->nv, h->sm_count), MS_RZ, op, s);
 }
 
 // one lockstep PCG iteration of the correction (body of the loop graph)
@@ -320,18 +321,21 @@ int mv_iteration(amgt_amg *h, MultiRhs *mr, cudaStream_t s, int use_cond, cudaGr
 {
     const int nv = mr->nv;
     const long long n = h->n0;
-    AMGT_TRY(apply(h, h->prm.inner_prec0, &h->lv[0].A, 1.0, mr->p, nv, 0.0, mr->q, s));
-    AMGT_TRY(mv_dot(h, mr, mr->p, mr->q, MS_PQ, MOP_ALPHA, s));
+    MvArgs a{};
+    a.X = mr->p;
+    a.Y = mr->q;
+    a.part = mr->part;
+    AMGT_TRY(mv_apply(h->prm.inner_prec0, MV_DOT, &h->lv[0].A, nv, a, s, h->sm_count));
+    AMGT_TRY(mv_reduce(h, mr, mv_apply_grid(&h->lv[0].A, nv, h->sm_count), MS_PQ, MOP_ALPHA, s));
     AMGT_LAUNCH_PDL(mv_axpy2_dot_kernel, kMvGrid, kMvThreads, 0, s, n, nv, (const double *)mr->scal,
                     (const double *)mr->p, (const double *)mr->q, mr->d, mr->r, mr->part);
-    AMGT_LAUNCH_PDL(mv_reduce_kernel, 1, 1024, 0, s, (const double *)mr->part, kMvGrid, nv, mr->scal, (int)MS_RR,
-                    (int)MOP_RR_TEST, h->prm.inner_tol);
-    AMGT_TRY(mv_cycle(h, mr, mr->r, mr->z, s));
-    AMGT_TRY(mv_dot(h, mr, mr->r, mr->z, MS_RZ, MOP_BETA, s));
+    AMGT_TRY(mv_reduce(h, mr, kMvGrid, MS_RR, MOP_RR_TEST, s));
+    AMGT_TRY(mv_cycle(h, mr, mr->r, mr->z, true, s));
+    AMGT_TRY(mv_cycle_dot(h, mr, mr->r, mr->z, MOP_BETA, s));
     AMGT_LAUNCH_PDL(mv_xpby_kernel, mv_grid(n, h->sm_count), kMvThreads, 0, s, n, nv, (const double *)mr->z,
                     (const double *)mr->scal, mr->p);
     count_launch();
-    mv_continue_kernel<<<1, 1, 0, s>>>(cond, use_cond, nv, mr->scal, mr->cnt, h->prm.max_iter, mr->cnt + 33);
+    mv_continue_kernel<<<1, 32, 0, s>>>(cond, use_cond, nv, mr->scal, mr->cnt, h->prm.max_iter, mr->cnt + 33);
     AMGT_CUDA_TRY(cudaGetLastError());
     return AMGT_OK;
 }
@@ -444,8 +448,11 @@ extern "C" int amgt_amg_solve_multi(amgt_amg *h, int nrhs, const double *B, doub
     int seen = 0;
     for (int outer = 0; outer <= h->prm.max_outer; ++outer) {
         // fp64 residual R = B - A X (8-byte values, CUDA cores)
-        AMGT_LAUNCH_PDL(mv_copy_kernel, grid_for(256, cnt_all, h->sm_count, 8), 256, 0, s, cnt_all, B, mr->res);
-        AMGT_TRY(spmm_rowmajor(AMGT_DOUBLE, 0, 8, &v0.A, -1.0, X, nv, 1.0, mr->res, s, h->sm_count));
+        MvArgs ra{};
+        ra.X = X;
+        ra.F = B;
+        ra.Y = mr->res;
+        AMGT_TRY(mv_apply(AMGT_DOUBLE, MV_RESID, &v0.A, nv, ra, s, h->sm_count));
         AMGT_TRY(mv_dot(h, mr, mr->res, mr->res, MS_RR, MOP_STORE, s));
         AMGT_CUDA_TRY(cudaMemcpyAsync(mr->pinned, mr->scal, sizeof(double) * 64, cudaMemcpyDeviceToHost, s));
         AMGT_CUDA_TRY(cudaMemcpyAsync(mr->pinned + 64, mr->cnt, sizeof(int) * 34, cudaMemcpyDeviceToHost, s));
@@ -476,8 +483,8 @@ extern "C" int amgt_amg_solve_multi(amgt_amg *h, int nrhs, const double *B, doub
         AMGT_LAUNCH_PDL(mv_copy_kernel, grid_for(256, cnt_all, h->sm_count, 8), 256, 0, s, cnt_all,
                         (const double *)mr->res, mr->r);
         AMGT_TRY(mv_dot(h, mr, mr->r, mr->r, MS_RR0, MOP_START, s));
-        AMGT_TRY(mv_cycle(h, mr, mr->r, mr->z, s));
-        AMGT_TRY(mv_dot(h, mr, mr->r, mr->z, MS_RZ, MOP_STORE, s));
+        AMGT_TRY(mv_cycle(h, mr, mr->r, mr->z, true, s));
+        AMGT_TRY(mv_cycle_dot(h, mr, mr->r, mr->z, MOP_STORE, s));
         AMGT_LAUNCH_PDL(mv_copy_kernel, grid_for(256, cnt_all, h->sm_count, 8), 256, 0, s, cnt_all,
                         (const double *)mr->z, mr->p);
         bool done = false;

@@ -237,7 +237,7 @@ AMGT_API int amgt_spmm(int prec, double alpha, const amgt_bsr *A, int nvec,
  * beta = 1 gives an fp64 residual of products computed on the tensor
  * cores).  prec DOUBLE: fp64 on the CUDA cores.  engine CUDA_CORE: a warp
  * per block row, a lane per right-hand side.  engine AUTO: amgt_autotune's
- * choice for (A, prec, nvec), else the tensor cores with 8 warps per CTA.
+ * choice for (A, prec, nvec), else the CUDA cores.
  * An fp32 request on a matrix whose exact fp16 shadow holds every value
  * reads that shadow.  Never blocks the host. */
 #define AMGT_ENGINE_AUTO 0
