@@ -10,6 +10,7 @@
 // bitmap table.  Two passes: count (sorts, keeps the sorted pairs in
 // scratch, sizes the arrays with one host read-back), then fill (block
 // columns, bitmaps, zero-padded values from the kept pairs).
+#include <algorithm>
 #include <atomic>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -74,7 +75,7 @@ __device__ __forceinline__ BlockRowRange block_row_range(const int *ia, int m, i
 // or reports the bad index).  27-point operators (108 entries and about 27
 // block columns per block row) stay on this path.
 constexpr int kStWarps = 4;
-constexpr int kStCap = 1024;    // entries of a warp's 32 block rows held in shared memory
+constexpr int kStCap = 1024;    // entries of a warp's block rows held in shared memory
 constexpr int kStRowMax = 128;  // entries of a block row on this path
 
 __global__ void __launch_bounds__(32 * kStWarps)
@@ -163,6 +164,121 @@ csr2bsr_count_sorted_kernel(int m, int n, const int *__restrict__ ia, const int 
             if (lane == 0) at = atomicAdd(nslow, __popc(left));
             at = __shfl_sync(FULL, at, 0);
             if (live && !ok) slow[at + __popc(left & ((1u << lane) - 1))] = b;
+        }
+        __syncwarp();  // the shared entries are reused by the next group
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long om = __shfl_xor_sync(FULL, wmax, o);
+        wmax = wmax > om ? wmax : om;
+        wsq += __shfl_xor_sync(FULL, wsq, o);
+    }
+    if (lane == 0 && wsq) {
+        atomicMax((unsigned long long *)&stats[0], wmax);
+        atomicAdd((unsigned long long *)&stats[1], wsq);
+    }
+}
+
+// The same pass for longer rows: four lanes per block row, lane q on CSR row
+// q.  The quad takes the lowest head of its 8 lists by two shuffles, each lane
+// gives its matching entries the rank, the lowest lane's first one the flag.
+// The columns of a warp's 8 block rows come into shared memory, and their
+// slot bytes leave from it, with coalesced accesses when they fit.
+// 27-point 96^3 (23.3 M entries): 209 us, bound by the merge's instructions;
+// one lane per block row, whose stage holds 1,024 entries of 32 block rows and
+// which reads longer ones entry by entry, took 343.  For short rows the quad
+// idles (7-point 128^3 BoomerAMG setup's conversions: 407 us against 225).
+__global__ void __launch_bounds__(32 * kStWarps)
+csr2bsr_count_quad_kernel(int m, int n, const int *__restrict__ ia, const int *__restrict__ ja, int brow,
+                            int *__restrict__ cnt, int *__restrict__ slow, int *__restrict__ nslow,
+                            unsigned char *__restrict__ slowf, int64_t *__restrict__ stats,
+                            unsigned char *__restrict__ slotb)
+{
+    constexpr int NONE = 0x7FFFFFFF;
+    __shared__ int scol[kStWarps][kStCap];
+    __shared__ unsigned char sslot[kStWarps][kStCap];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
+    const unsigned gmask = 0xFu << (lane & ~3);
+    int *sc = scol[warp];
+    unsigned char *ss = sslot[warp];
+    unsigned long long wmax = 0, wsq = 0;
+    const int ngroups = (brow + 7) / 8;
+    for (int gi = blockIdx.x * kStWarps + warp; gi < ngroups; gi += gridDim.x * kStWarps) {
+        const int b = gi * 8 + (lane >> 2), row = 4 * b + q;
+        const bool live = b < brow;
+        const int p = __ldg(ia + min(row, m)), pe = __ldg(ia + min(row + 1, m));
+        const int E0 = __shfl_sync(FULL, p, 0), E1 = __shfl_sync(FULL, pe, 31);
+        const bool staged = E1 - E0 <= kStCap;  // warp-uniform
+        if (staged)
+            for (int e = E0 + lane; e < E1; e += 32) sc[e - E0] = __ldg(ja + e);
+        __syncwarp();
+        const int nrow = __shfl_sync(FULL, pe, lane | 3) - __shfl_sync(FULL, p, lane & ~3);
+        bool ok = live && nrow <= kStRowMax;  // the same for the quad, as every break below
+        int u = 0;
+        if (ok) {
+            bool bad = false;
+            auto block_col = [&](int e) -> int {
+                const int col = staged ? sc[e - E0] : __ldg(ja + e);
+                if (col < 0 || col >= n) bad = true;
+                return col >> 2;
+            };
+            auto put = [&](int e, unsigned v) {
+                if (staged) ss[e - E0] = (unsigned char)v;
+                else slotb[e] = (unsigned char)v;
+            };
+            int t = p + 1;  // the rest of the row
+            int hc = p < pe ? block_col(p) : NONE, tc = t < pe ? block_col(t) : NONE;
+            ok = !__any_sync(gmask, bad);
+            while (ok) {
+                int mn = min(hc, tc);
+                mn = min(mn, __shfl_xor_sync(gmask, mn, 1));
+                mn = min(mn, __shfl_xor_sync(gmask, mn, 2));
+                if (mn == NONE) break;
+                if (u == 32) {  // a 33rd block column: slot bytes hold 0..31
+                    ok = false;
+                    break;
+                }
+                const unsigned hit = __ballot_sync(gmask, hc == mn || tc == mn);
+                unsigned lead = lane == __ffs(hit) - 1 ? 0x80u : 0u;
+                if (hc == mn) {
+                    put(p, u | lead);
+                    lead = 0;
+                    hc = NONE;
+                }
+                while (tc == mn) {
+                    put(t, u | lead);
+                    lead = 0;
+                    tc = NONE;
+                    if (++t < pe) {
+                        tc = block_col(t);
+                        if (tc < mn) {  // unsorted
+                            bad = true;
+                            tc = NONE;
+                        }
+                    }
+                }
+                ++u;
+            }
+            if (__any_sync(gmask, bad)) ok = false;
+        }
+        __syncwarp();
+        if (staged)
+            for (int e = E0 + lane; e < E1; e += 32) slotb[e] = ss[e - E0];
+        if (live && q == 0) {
+            slowf[b] = ok ? 0 : 1;
+            if (ok) {
+                cnt[b] = u;
+                wmax = wmax > (unsigned long long)u ? wmax : (unsigned long long)u;
+                wsq += (unsigned long long)u * (unsigned long long)u;
+            }
+        }
+        const bool leave = live && !ok && q == 0;
+        const unsigned left = __ballot_sync(FULL, leave);
+        if (left) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(nslow, __popc(left));
+            at = __shfl_sync(FULL, at, 0);
+            if (leave) slow[at + __popc(left & ((1u << lane) - 1))] = b;
         }
         __syncwarp();  // the shared entries are reused by the next group
     }
@@ -420,7 +536,10 @@ csr2bsr_large_kernel(int m, int n, const int *__restrict__ ia, const int *__rest
 // blocks.  A block's bitmap is the OR of the 4 lanes' nibbles (shuffles in
 // the group), and the first entry of a column writes the block column.  A
 // warp takes 8 block rows at a time and first copies their entries (column,
-// value, slot byte) into shared memory with coalesced loads.
+// value, slot byte) into shared memory with coalesced loads, when they fit
+// the stage of `cap` entries (chosen from the mean row, up to kFsCapMax: a
+// 27-point operator's 864 fit; reading them entry by entry from global memory
+// took 429 us at 96^3, 286 staged).
 // With every block row on this path the pass can also write, from the
 // values it holds: the fp16 rounding of each stored value and the
 // exactness bits of exact_check_kernel (v16, flags), the fp32 rounding
@@ -428,7 +547,8 @@ csr2bsr_large_kernel(int m, int n, const int *__restrict__ ia, const int *__rest
 // summed as l1_norm_kernel sums it (blocks in order, |v0| + |v1| + |v2| +
 // |v3| per block; 1 / norm with l1_invert).
 constexpr int kFsWarps = 4;
-constexpr int kFsCap = 256;  // entries of a warp's 8 block rows held in shared memory
+constexpr int kFsCapMin = 256, kFsCapMax = 1024;  // entries of a warp's 8 block rows held in shared memory
+constexpr int kFsEntry = 13;                      // bytes of a staged entry
 
 struct FillExtras {
     __half *v16;                // nullable
@@ -442,31 +562,34 @@ __global__ void __launch_bounds__(32 * kFsWarps)
 csr2bsr_fill_sorted_kernel(int m, const int *__restrict__ ia, const int *__restrict__ ja,
                            const double *__restrict__ a, int brow, const unsigned char *__restrict__ slowf,
                            const int *__restrict__ bptr, int *__restrict__ bidx, uint16_t *__restrict__ bmap,
-                           double *__restrict__ bval, const unsigned char *__restrict__ slotb, FillExtras fx)
+                           double *__restrict__ bval, const unsigned char *__restrict__ slotb, FillExtras fx, int cap)
 {
     bool not32 = false, not16 = false;
-    __shared__ double sval[kFsWarps][kFsCap];
-    __shared__ int scol[kFsWarps][kFsCap];
-    __shared__ unsigned char sslot[kFsWarps][kFsCap];
+    extern __shared__ double fs_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
+    double *sval = fs_smem + warp * cap;
+    int *scol = reinterpret_cast<int *>(fs_smem + kFsWarps * cap) + warp * cap;
+    unsigned char *sslot = reinterpret_cast<unsigned char *>(fs_smem + kFsWarps * cap + kFsWarps * cap / 2) + warp * cap;
     const unsigned gmask = 0xFu << (lane & ~3);
     const int nwg = (brow + 7) / 8;
     for (int wg = blockIdx.x * kFsWarps + warp; wg < nwg; wg += gridDim.x * kFsWarps) {
         const int b0 = 8 * wg;
         const int E0 = __ldg(ia + 4 * b0), E1 = __ldg(ia + min(4 * (b0 + 8), m));
-        const bool staged = E1 - E0 <= kFsCap;  // warp-uniform
-        if (staged)
+        const bool staged = E1 - E0 <= cap;  // warp-uniform
+        if (staged) {
+#pragma unroll 4
             for (int e = E0 + lane; e < E1; e += 32) {
-                scol[warp][e - E0] = __ldg(ja + e);
-                sval[warp][e - E0] = __ldg(a + e);
-                sslot[warp][e - E0] = __ldg(slotb + e);
+                scol[e - E0] = __ldg(ja + e);
+                sval[e - E0] = __ldg(a + e);
+                sslot[e - E0] = __ldg(slotb + e);
             }
+        }
         __syncwarp();
         auto entry = [&](int p, int &sb, int &c, double &v) {
             if (staged) {
-                sb = sslot[warp][p - E0];
-                c = scol[warp][p - E0];
-                v = sval[warp][p - E0];
+                sb = sslot[p - E0];
+                c = scol[p - E0];
+                v = sval[p - E0];
             } else {
                 sb = __ldg(slotb + p);
                 c = __ldg(ja + p);
@@ -988,8 +1111,14 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
     if (brow > 0) {
         // slow-row list behind the large-row list (2 brow ints)
         int *slow = large + brow, *nslow = (int *)&stats[4];
-        AMGT_LAUNCH(csr2bsr_count_sorted_kernel, grid_for(32 * kStWarps, brow, st->sm_count, 12), 32 * kStWarps, 0,
-                    s, m, n, A->i, A->j, brow, cnt, slow, nslow, slowf, stats, slotb);
+        // a quad per block row once 32 mean block rows overflow the stage of
+        // the lane-per-block-row form
+        if (128LL * A->num_nonzeros > (long long)kStCap * m)
+            AMGT_LAUNCH(csr2bsr_count_quad_kernel, grid_for(8 * kStWarps, brow, st->sm_count, 11), 32 * kStWarps, 0,
+                        s, m, n, A->i, A->j, brow, cnt, slow, nslow, slowf, stats, slotb);
+        else
+            AMGT_LAUNCH(csr2bsr_count_sorted_kernel, grid_for(32 * kStWarps, brow, st->sm_count, 12), 32 * kStWarps,
+                        0, s, m, n, A->i, A->j, brow, cnt, slow, nslow, slowf, stats, slotb);
         AMGT_LAUNCH(csr2bsr_count_kernel, 2 * st->sm_count, 32 * kCvtWarps, 0, s, m, n, A->i, A->j, brow, slow,
                     nslow, cnt, large, stats, st->err, sorted, slotb);
         AMGT_LAUNCH(csr2bsr_large_kernel<false>, 2 * st->sm_count, kLargeThreads, 2 * kWin * sizeof(uint32_t), s,
@@ -1035,9 +1164,16 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
     }
     if (brow > 0) {
         const int *slow = large + brow, *nslow = (const int *)&stats[4];
-        AMGT_LAUNCH(csr2bsr_fill_sorted_kernel, grid_for(8 * kFsWarps, brow, st->sm_count, 16), 32 * kFsWarps, 0, s,
-                    m, A->i, A->j,
-                    A->data, brow, slowf, out->blcPtr, out->blcIdx, out->blcMap, out->blcVal, slotb, fx);
+        // the stage: a quarter more than the mean of 8 block rows
+        const long long want = 40LL * A->num_nonzeros / m;
+        const int cap = (int)std::min<long long>(kFsCapMax, std::max<long long>(kFsCapMin, (want + 15) & ~15LL));
+        const int fs_bytes = kFsWarps * cap * kFsEntry;
+        if (fs_bytes > 48 * 1024)
+            AMGT_CUDA_TRY(cudaFuncSetAttribute(csr2bsr_fill_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               fs_bytes));
+        AMGT_LAUNCH(csr2bsr_fill_sorted_kernel, grid_for(8 * kFsWarps, brow, st->sm_count, 16), 32 * kFsWarps,
+                    fs_bytes, s, m, A->i, A->j, A->data, brow, slowf, out->blcPtr, out->blcIdx, out->blcMap,
+                    out->blcVal, slotb, fx, cap);
         AMGT_LAUNCH(csr2bsr_fill_kernel, 2 * st->sm_count, 32 * kCvtWarps, 0, s, m, n, A->i, A->j, A->data, brow,
                     slow, nslow, out->blcPtr, out->blcIdx, out->blcMap, out->blcVal, sorted, slotb, st->err);
         AMGT_LAUNCH(csr2bsr_large_kernel<true>, 2 * st->sm_count, kLargeThreads, 2 * kWin * sizeof(uint32_t), s, m,
