@@ -662,7 +662,7 @@ void destroy_handle(amgt_amg *h, cudaStream_t s)
     free_ptr(h->gm_j, s);
     if (h->mr) free_multi_rhs(h->mr, s);
     if (h->batch) free_batch(h->batch, s);
-    if (h->graph_stream) cudaStreamDestroy(h->graph_stream);
+    stream_put(h->graph_stream);
     free_ptr(h->loop_it, s);
     free_ptr(h->loop_rr, s);
     // loop_pinned and mr_pinned live inside the one pinned block h->pinned
@@ -894,7 +894,7 @@ int build_loop_graph(amgt_amg *h, double *x)
         cudaGraphExecDestroy(h->loop);
         h->loop = nullptr;
     }
-    if (!h->graph_stream) AMGT_CUDA_TRY(cudaStreamCreateWithFlags(&h->graph_stream, cudaStreamNonBlocking));
+    if (!h->graph_stream) AMGT_TRY(stream_get(&h->graph_stream));
     if (!h->loop_it || !h->loop_rr) return AMGT_ERR_INVALID;  // allocated by the setup
     if (!h->loop_pinned) return AMGT_ERR_INVALID;  // allocated by the setup
     cudaGraph_t g = nullptr;
@@ -950,7 +950,7 @@ int build_graph(amgt_amg *h, double *x)
         cudaGraphExecDestroy(h->graph);
         h->graph = nullptr;
     }
-    if (!h->graph_stream) AMGT_CUDA_TRY(cudaStreamCreateWithFlags(&h->graph_stream, cudaStreamNonBlocking));
+    if (!h->graph_stream) AMGT_TRY(stream_get(&h->graph_stream));
     cudaGraph_t g = nullptr;
     AMGT_CUDA_TRY(cudaStreamBeginCapture(h->graph_stream, cudaStreamCaptureModeThreadLocal));
     const uint64_t c0 = amgt_kernel_launch_count();
@@ -997,7 +997,7 @@ int gm_iteration(amgt_amg *h, cudaStream_t s, int use_cond, cudaGraphConditional
 int build_gm_loop(amgt_amg *h)
 {
     if (h->gm_loop) return AMGT_OK;
-    if (!h->graph_stream) AMGT_CUDA_TRY(cudaStreamCreateWithFlags(&h->graph_stream, cudaStreamNonBlocking));
+    if (!h->graph_stream) AMGT_TRY(stream_get(&h->graph_stream));
     cudaGraph_t g = nullptr;
     AMGT_CUDA_TRY(cudaGraphCreate(&g, 0));
     cudaGraphConditionalHandle cond;
@@ -1226,7 +1226,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
     }
     // the second stream starts after everything the caller queued on `s`
     // before this call (the inputs may still be arriving there)
-    if (L > 1 && (cudaStreamCreateWithFlags(&nx.s2, cudaStreamNonBlocking) != cudaSuccess ||
+    if (L > 1 && (stream_get(&nx.s2) != AMGT_OK ||
                   cudaEventCreateWithFlags(&nx.p_ready[0], cudaEventDisableTiming) != cudaSuccess ||
                   cudaEventCreateWithFlags(&nx.p_ready[1], cudaEventDisableTiming) != cudaSuccess ||
                   cudaEventCreateWithFlags(&nx.r_ready[0], cudaEventDisableTiming) != cudaSuccess ||
@@ -1581,7 +1581,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
     free_ptr(xflags, s);
     pm.mark(3, s);
     pm.accumulate(h->setup_ms);  // waits for the setup's last work
-    if (nx.s2) cudaStreamDestroy(nx.s2);
+    stream_put(nx.s2);
     for (int i = 0; i < 2; ++i) {
         if (nx.p_ready[i]) cudaEventDestroy(nx.p_ready[i]);
         if (nx.r_ready[i]) cudaEventDestroy(nx.r_ready[i]);
@@ -1591,7 +1591,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
 fail:
     if (nx.s2) {  // its conversions may still use arrays the handle frees
         cudaStreamSynchronize(nx.s2);
-        cudaStreamDestroy(nx.s2);
+        stream_put(nx.s2);
     }
     cudaStreamSynchronize(s);  // no kernel of this setup in flight
     if (xflags) free_ptr(xflags, s);

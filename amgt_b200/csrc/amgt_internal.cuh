@@ -212,6 +212,21 @@ int exclusive_scan_i64(const int64_t *in, int64_t *out, int n, cudaStream_t s);
 // returns a pointer to the pinned slots (valid until the thread's next
 // read_back on the device).
 int read_back(const int64_t *dev, int count, cudaStream_t s, const int64_t **host);
+// The same for up to 8 scattered device values, int (wide 0, sign-extended)
+// or int64: host[i] is item i.
+struct ReadList {
+    struct Item {
+        const void *p;
+        int wide;
+    } item[8];
+    int n = 0;
+    void add(const int *p) { item[n++] = Item{p, 0}; }
+    void add(const int64_t *p) { item[n++] = Item{p, 1}; }
+};
+int read_back_items(const ReadList &items, cudaStream_t s, const int64_t **host);
+// Non-blocking streams of the library's own, kept for reuse (bounded).
+int stream_get(cudaStream_t *out);
+void stream_put(cudaStream_t s);
 // Pinned host blocks for the handles' read-back slots, from a library cache
 // reused across handles (cudaMallocHost only on a miss); pinned_put returns
 // a block to the cache, amgt_trim_pool frees the cached ones.

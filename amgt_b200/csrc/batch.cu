@@ -242,7 +242,7 @@ int b_iteration(amgt_amg *h, Batch *b, double *x, cudaStream_t s, int use_cond, 
 int build_b_loop(amgt_amg *h, Batch *b, double *x)
 {
     if (b->loop) return AMGT_OK;
-    if (!h->graph_stream) AMGT_CUDA_TRY(cudaStreamCreateWithFlags(&h->graph_stream, cudaStreamNonBlocking));
+    if (!h->graph_stream) AMGT_TRY(stream_get(&h->graph_stream));
     cudaGraph_t g = nullptr;
     AMGT_CUDA_TRY(cudaGraphCreate(&g, 0));
     cudaGraphConditionalHandle cond;

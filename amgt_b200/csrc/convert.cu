@@ -1086,7 +1086,7 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
     unsigned char *slotb = nullptr;        // per entry of shorter rows: block slot | first-of-column flag
     int rc = AMGT_OK;
     const int64_t *h = nullptr;
-    int nb = 0;
+    int nb = 0, h_large = 0, h_slow = 0;  // blocks; block rows left to the large-row and warp kernels
     FillExtras fx{nullptr, nullptr, nullptr, nullptr, 0};
     bool all_sorted = false;  // no block row left to the warp or large-row kernels
     static std::atomic<bool> smem_set[64];  // per device: the large-row kernels' shared-memory opt-in
@@ -1101,13 +1101,13 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
     }
     // stats: [0] longest block row, [1] sum of squares, [2] block count,
     // [3] large-row count (int), [4] slow-row count (int)
-    if ((rc = alloc_n(&out->blcPtr, brow + 1, s)) || (rc = alloc_n(&cnt, brow + 1, s)) ||
-        (rc = alloc_n(&large, 2 * (size_t)brow, s)) || (rc = alloc_n(&stats, 5, s)) ||
+    if ((rc = alloc_n(&out->blcPtr, brow + 1, s)) || (rc = alloc_n(&stats, 5 + ((size_t)brow + 2) / 2, s)) ||
+        (rc = alloc_n(&large, 2 * (size_t)brow, s)) ||
         (rc = alloc_n(&sorted, (size_t)A->num_nonzeros, s)) ||
         (rc = alloc_n(&slotb, (size_t)A->num_nonzeros, s)) || (rc = alloc_n(&slowf, (size_t)brow, s)))
         goto fail;
-    AMGT_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(int64_t) * 5, s));
-    AMGT_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * (brow + 1), s));
+    cnt = reinterpret_cast<int *>(stats + 5);  // the counts behind the statistics: one clear
+    AMGT_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(int64_t) * 5 + sizeof(int) * ((size_t)brow + 1), s));
     if (brow > 0) {
         // slow-row list behind the large-row list (2 brow ints)
         int *slow = large + brow, *nslow = (int *)&stats[4];
@@ -1125,11 +1125,20 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
                     m, n, A->i, A->j, A->data, large, stats, cnt, nullptr, nullptr, nullptr, nullptr, stats);
     }
     if ((rc = exclusive_scan_int(cnt, out->blcPtr, brow + 1, s))) goto fail;
-    AMGT_CUDA_TRY(cudaMemcpyAsync(&stats[2], out->blcPtr + brow, sizeof(int), cudaMemcpyDeviceToDevice, s));
     if (between && (rc = between(ctx))) goto fail;
-    if ((rc = read_back(stats, 5, s, &h))) goto fail;
+    {
+        ReadList rl;
+        rl.add(stats);
+        rl.add(stats + 1);
+        rl.add(out->blcPtr + brow);
+        rl.add((const int *)&stats[3]);
+        rl.add((const int *)&stats[4]);
+        if ((rc = read_back_items(rl, s, &h))) goto fail;
+    }
     nb = (int)h[2];
-    all_sorted = h[3] == 0 && h[4] == 0;
+    h_large = (int)h[3];
+    h_slow = (int)h[4];
+    all_sorted = h_large == 0 && h_slow == 0;
     out->max_blc_per_row = (int)h[0];
     {
         const double S2 = (double)h[1];
@@ -1174,13 +1183,14 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
         AMGT_LAUNCH(csr2bsr_fill_sorted_kernel, grid_for(8 * kFsWarps, brow, st->sm_count, 16), 32 * kFsWarps,
                     fs_bytes, s, m, A->i, A->j, A->data, brow, slowf, out->blcPtr, out->blcIdx, out->blcMap,
                     out->blcVal, slotb, fx, cap);
-        AMGT_LAUNCH(csr2bsr_fill_kernel, 2 * st->sm_count, 32 * kCvtWarps, 0, s, m, n, A->i, A->j, A->data, brow,
+        if (h_slow > 0)
+            AMGT_LAUNCH(csr2bsr_fill_kernel, 2 * st->sm_count, 32 * kCvtWarps, 0, s, m, n, A->i, A->j, A->data, brow,
                     slow, nslow, out->blcPtr, out->blcIdx, out->blcMap, out->blcVal, sorted, slotb, st->err);
-        AMGT_LAUNCH(csr2bsr_large_kernel<true>, 2 * st->sm_count, kLargeThreads, 2 * kWin * sizeof(uint32_t), s, m,
+        if (h_large > 0)
+            AMGT_LAUNCH(csr2bsr_large_kernel<true>, 2 * st->sm_count, kLargeThreads, 2 * kWin * sizeof(uint32_t), s, m,
                     n, A->i, A->j, A->data, large, stats, nullptr, out->blcPtr, out->blcIdx, out->blcMap, out->blcVal,
                     nullptr);
     }
-    free_ptr(cnt, s);
     free_ptr(large, s);
     free_ptr(stats, s);
     free_ptr(sorted, s);
@@ -1188,7 +1198,6 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
     free_ptr(slowf, s);
     return AMGT_OK;
 fail:
-    free_ptr(cnt, s);
     free_ptr(large, s);
     free_ptr(stats, s);
     free_ptr(sorted, s);

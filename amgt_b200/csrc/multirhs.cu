@@ -343,7 +343,7 @@ int mv_iteration(amgt_amg *h, MultiRhs *mr, cudaStream_t s, int use_cond, cudaGr
 int build_mv_loop(amgt_amg *h, MultiRhs *mr)
 {
     if (mr->loop) return AMGT_OK;
-    if (!h->graph_stream) AMGT_CUDA_TRY(cudaStreamCreateWithFlags(&h->graph_stream, cudaStreamNonBlocking));
+    if (!h->graph_stream) AMGT_TRY(stream_get(&h->graph_stream));
     cudaGraph_t g = nullptr;
     AMGT_CUDA_TRY(cudaGraphCreate(&g, 0));
     cudaGraphConditionalHandle cond;

@@ -314,20 +314,94 @@ int check_device_error(cudaStream_t s)
     return AMGT_OK;
 }
 
-int read_back(const int64_t *dev, int count, cudaStream_t s, const int64_t **host)
+// One warp writes the slots and the error word straight into the host's
+// pinned staging: one launch where each copy is an API call and about 3 us of
+// the stream (a 2D 128^2 setup reads back 29 times, 57 copies and 44 device
+// copies that gathered their sources).
+__global__ void read_back_kernel(const int64_t *__restrict__ dev, int count, ReadList items,
+                                 const int *__restrict__ err, int64_t *__restrict__ out)
+{
+    for (int i = threadIdx.x; i < count; i += blockDim.x) out[i] = dev[i];
+    if ((int)threadIdx.x < items.n) {
+        const ReadList::Item &it = items.item[threadIdx.x];
+        out[count + threadIdx.x] =
+            it.wide ? *static_cast<const int64_t *>(it.p) : (int64_t)*static_cast<const int *>(it.p);
+    }
+    if (threadIdx.x == 0) out[kErrSlot] = *err;
+}
+
+static int read_back_launch(const int64_t *dev, int count, const ReadList &items, cudaStream_t s, const int64_t **host)
 {
     DeviceState *st;
     AMGT_TRY(device_state(&st));
-    if (count > kErrSlot) return AMGT_ERR_INVALID;
+    if (count < 0 || count + items.n > kErrSlot) return AMGT_ERR_INVALID;
     int64_t *pin;
     AMGT_TRY(staging(&pin));
     pin[kErrSlot] = 0;
-    AMGT_CUDA_TRY(cudaMemcpyAsync(pin, dev, sizeof(int64_t) * count, cudaMemcpyDeviceToHost, s));
-    AMGT_CUDA_TRY(cudaMemcpyAsync(&pin[kErrSlot], st->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AMGT_LAUNCH(read_back_kernel, 1, 32, 0, s, dev, count, items, (const int *)st->err, pin);
     AMGT_CUDA_TRY(cudaStreamSynchronize(s));
     *host = pin;
     return AMGT_OK;
 }
+
+int read_back_items(const ReadList &items, cudaStream_t s, const int64_t **host)
+{
+    return read_back_launch(nullptr, 0, items, s, host);
+}
+
+int read_back(const int64_t *dev, int count, cudaStream_t s, const int64_t **host)
+{
+    return read_back_launch(dev, count, ReadList{}, s, host);
+}
+
+// Streams of the library's own (the setup's second stream, the solvers'
+// capture streams): creating and destroying one costs about 0.1 ms each, so
+// up to kStreamsKept per device are kept when a handle gives them back, until
+// amgt_trim_pool or exit.
+static constexpr size_t kStreamsKept = 16;
+static std::mutex g_stream_mu;
+static std::vector<cudaStream_t> g_streams[kMaxDevices];
+
+int stream_get(cudaStream_t *out)
+{
+    int dev = 0;
+    AMGT_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < kMaxDevices) {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        if (!g_streams[dev].empty()) {
+            *out = g_streams[dev].back();
+            g_streams[dev].pop_back();
+            return AMGT_OK;
+        }
+    }
+    AMGT_CUDA_TRY(cudaStreamCreateWithFlags(out, cudaStreamNonBlocking));
+    return AMGT_OK;
+}
+
+void stream_put(cudaStream_t s)
+{
+    if (!s) return;
+    int dev = 0;
+    // the stream's own device, which may not be the current one
+    if (cudaStreamGetDevice(s, &dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        if (g_streams[dev].size() < kStreamsKept) {
+            g_streams[dev].push_back(s);
+            return;
+        }
+    }
+    cudaGetLastError();
+    cudaStreamDestroy(s);
+}
+
+static void streams_trim(int dev)
+{
+    std::lock_guard<std::mutex> lk(g_stream_mu);
+    if (dev < 0 || dev >= kMaxDevices) return;
+    for (cudaStream_t s : g_streams[dev]) cudaStreamDestroy(s);
+    g_streams[dev].clear();
+}
+
 
 // ------------------------------------------------------------------ scans
 // Exclusive sum of up to kSmallScan entries in one launch of one CTA
@@ -471,6 +545,7 @@ int amgt_trim_pool(size_t keep_bytes)
     flush_cache(dev);
     AMGT_CUDA_TRY(cudaDeviceSynchronize());
     pinned_trim();
+    streams_trim(dev);
     AMGT_CUDA_TRY(cudaMemPoolTrimTo(pool, keep_bytes));
     return AMGT_OK;
 }

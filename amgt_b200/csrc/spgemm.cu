@@ -2262,10 +2262,10 @@ int spgemm_impl(int prec, const amgt_bsr *A, const amgt_bsr *B, amgt_bsr *C, amg
                             ? (long long)A->blc_num * (long long)B->max_blc_per_row
                             : -1;
         if (cap < 0 || cap > (32LL << 20)) {
-            AMGT_CUDA_TRY(cudaMemcpyAsync(&stats[2], ub_off + brA, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
-            if ((rc = read_back(stats, 4, s, &h))) goto fail;
-            cap = h[2];
-            AMGT_CUDA_TRY(cudaMemsetAsync(&stats[2], 0, sizeof(int64_t), s));
+            ReadList rl;
+            rl.add(ub_off + brA);
+            if ((rc = read_back_items(rl, s, &h))) goto fail;
+            cap = h[0];
         }
         // pattern keys, bitmaps and pair slots in one allocation
         const size_t o_map = align256(4 * (size_t)cap), o_slot = o_map + align256(2 * (size_t)cap),
@@ -2293,14 +2293,20 @@ int spgemm_impl(int prec, const amgt_bsr *A, const amgt_bsr *B, amgt_bsr *C, amg
                     32 * kSymWarps, 0, s, m, brA, A->blcPtr, A->blcIdx, A->blcMap, B->blcPtr, B->blcIdx, B->blcMap,
                     ccnt, csrcnt, large, stats, ub_off, skey, smap, nullptr, nullptr, medium, nmedium, pslot,
                     st->err);
-        AMGT_LAUNCH((spgemm_symbolic_hashed_kernel<kSymCap, 2>), 9 * st->sm_count, 64, 0, s, m, A->blcPtr,
+        // no row can hold more pairs than the longest A row times the longest B
+        // row: the longer rows' kernels run only when that allows any
+        const long long longest = A->max_blc_per_row > 0 && B->max_blc_per_row > 0
+                                      ? (long long)A->max_blc_per_row * B->max_blc_per_row
+                                      : 1LL << 62;
+        if (longest > 256)
+            AMGT_LAUNCH((spgemm_symbolic_hashed_kernel<kSymCap, 2>), 9 * st->sm_count, 64, 0, s, m, A->blcPtr,
                     A->blcIdx, A->blcMap, B->blcPtr, B->blcIdx, B->blcMap, ccnt, csrcnt, stats, ub_off, skey, smap,
                     medium, nmedium, large, (int *)&stats[3], pslot, st->err);
-        AMGT_LAUNCH(spgemm_symbolic_large_kernel, 6 * st->sm_count, kSymLargeThreads, 0, s, m, A->blcPtr, A->blcIdx,
+        if (longest > kSymCap)
+            AMGT_LAUNCH(spgemm_symbolic_large_kernel, 6 * st->sm_count, kSymLargeThreads, 0, s, m, A->blcPtr, A->blcIdx,
                     A->blcMap, B->blcPtr, B->blcIdx, B->blcMap, large, stats, ccnt, csrcnt, ub_off, skey, smap);
     }
     if ((rc = exclusive_scan_int(ccnt, C->blcPtr, brA + 1, s))) goto fail;
-    AMGT_CUDA_TRY(cudaMemcpyAsync(&stats[2], C->blcPtr + brA, sizeof(int), cudaMemcpyDeviceToDevice, s));
     // CSR row pointer of C (into Ccsr->i, or a temporary when only the
     // nonzero count is wanted)
     if (Ccsr) {
@@ -2314,15 +2320,22 @@ int spgemm_impl(int prec, const amgt_bsr *A, const amgt_bsr *B, amgt_bsr *C, amg
         csr_i = csr_tmp;
     }
     if ((rc = exclusive_scan_int(csrcnt, csr_i, m + 1, s))) goto fail;
-    AMGT_CUDA_TRY(cudaMemcpyAsync((int *)&stats[2] + 1, csr_i + m, sizeof(int), cudaMemcpyDeviceToDevice, s));
     if (between && (rc = between(ctx))) goto fail;
     // the exact pair count rides along (it sizes the gathered numeric's lists)
-    AMGT_CUDA_TRY(cudaMemcpyAsync(&stats[4], ub_off + brA, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
-    if ((rc = read_back(stats, 5, s, &h))) goto fail;
-    npairs = h[4];
-    nbC = (int)(h[2] & 0xFFFFFFFF);
-    nlarge = (int)(h[3] & 0xFFFFFFFF);
-    nnzC = (int)(h[2] >> 32);
+    {
+        ReadList rl;
+        rl.add(stats);
+        rl.add(stats + 1);
+        rl.add(C->blcPtr + brA);
+        rl.add(csr_i + m);
+        rl.add((const int *)&stats[3]);
+        rl.add(ub_off + brA);
+        if ((rc = read_back_items(rl, s, &h))) goto fail;
+    }
+    nbC = (int)h[2];
+    nnzC = (int)h[3];
+    nlarge = (int)h[4];
+    npairs = h[5];
     C->max_blc_per_row = (int)h[0];
     {
         const double avg = brA ? (double)nbC / brA : 0.0;
