@@ -84,11 +84,14 @@ __global__ void __launch_bounds__(kDotThreads) reduce_kernel(const double *__res
     }
 }
 
-// x += alpha p; r -= alpha q; partials of r . r
+// x += alpha p; r -= alpha q; partials of r . r; with u, the cycle's first
+// sweep from a zero guess on the new r (jacobi_zero_kernel's arithmetic)
 __global__ void __launch_bounds__(kDotThreads) axpy2_dot_kernel(long long n, const double *__restrict__ scal,
                                                                const double *__restrict__ p,
                                                                const double *__restrict__ q, double *__restrict__ x,
-                                                               double *__restrict__ r, double *__restrict__ part)
+                                                               double *__restrict__ r, double *__restrict__ part,
+                                                               const double *__restrict__ inv_l1, double w,
+                                                               double *__restrict__ u)
 {
     grid_dependency_wait();
     __shared__ double sred[kDotThreads / 32];
@@ -99,6 +102,7 @@ __global__ void __launch_bounds__(kDotThreads) axpy2_dot_kernel(long long n, con
         const double ri = r[i] - alpha * q[i];
         r[i] = ri;
         s += ri * ri;
+        if (u) u[i] = w * ri * inv_l1[i];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
@@ -541,7 +545,8 @@ __global__ void __launch_bounds__(kDotThreads) gm_givens_kernel(cudaGraphConditi
 
 // V_j = vin = w / ||w|| (j already advanced)
 __global__ void gm_scale_kernel(long long n, const double *__restrict__ w, const int *__restrict__ jdev, int m,
-                                const double *__restrict__ gm, float *__restrict__ V, double *__restrict__ vin)
+                                const double *__restrict__ gm, float *__restrict__ V, double *__restrict__ vin,
+                                const double *__restrict__ inv_l1, double weight, double *__restrict__ u)
 {
     grid_dependency_wait();
     const int j = *jdev;
@@ -552,6 +557,7 @@ __global__ void gm_scale_kernel(long long n, const double *__restrict__ w, const
         const float f = (float)v;
         vj[e] = f;
         vin[e] = (double)f;  // the cycle sees the stored basis vector
+        if (u) u[e] = weight * (double)f * inv_l1[e];  // its first sweep from a zero guess
     }
 }
 
@@ -580,13 +586,15 @@ __global__ void gm_start_kernel(int m, const double *__restrict__ scal, int slot
 }
 
 __global__ void gm_scale_first_kernel(long long n, const double *__restrict__ r, int m, const double *__restrict__ gm,
-                                      float *__restrict__ V, double *__restrict__ vin)
+                                      float *__restrict__ V, double *__restrict__ vin,
+                                      const double *__restrict__ inv_l1, double weight, double *__restrict__ u)
 {
     const double inv = gm[GmLayout{m}.slot() + GM_INVH];
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
         const float f = (float)(r[e] * inv);
         V[e] = f;
         vin[e] = (double)f;
+        if (u) u[e] = weight * (double)f * inv_l1[e];
     }
 }
 
@@ -788,20 +796,20 @@ int level_shadow(amgt_bsr *A, int prec, amgt_stream_t stream)
     return amgt_bsr_make_shadow(A, prec, stream);
 }
 
-// z = M f: one V(1,1) cycle
-int cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s)
+// z = M f: one V(1,1) cycle; have_u: level 0's sweep from a zero guess on
+// rhs0 is in lv[0].u already (the kernel that made rhs0 wrote it)
+int cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s, bool have_u = false)
 {
     auto &lv = h->lv;
     const int L = (int)lv.size();
     const double w = h->prm.relax_weight;
     const bool pk = h->prm.packed != 0;
-    bool have_u = false;  // level l's sweep from a zero guess came with the restriction into it
     for (int l = 0; l < L - 1; ++l) {
         Level &v = lv[l];
         const double *f = (l == 0) ? rhs0 : v.f;
         if (!have_u)
             AMGT_LAUNCH_PDL(jacobi_zero_kernel, grid_n(h, v.n), 256, 0, s, (long long)v.n, f, v.inv_l1, w, v.u);
-        have_u = false;
+        have_u = false;  // else level l's sweep came with the restriction into it
         if (pk) {
             AMGT_TRY(pbsr_residual(&v.pA, f, v.u, v.t, s, h->sm_count));
             AMGT_TRY(pbsr_spmv(&v.pR, 1.0, v.t, 0.0, lv[l + 1].f, s, h->sm_count));
@@ -852,8 +860,36 @@ int dot(amgt_amg *h, const double *a, const double *b, int slot, int op, cudaStr
     return AMGT_OK;
 }
 
-// One PCG iteration after the first (q = A p ... p = z + beta p).
-int pcg_iteration(amgt_amg *h, double *x, cudaStream_t s)
+// ||r||^2 inside the loop graph: reduce_kernel's sum, then the iteration is
+// counted, ||r||^2 kept and the while condition set with the host loop's test
+// (relative residual above tol and fewer than max_iter iterations); the rest
+// of the body still runs once.
+__global__ void __launch_bounds__(kDotThreads) pcg_continue_kernel(cudaGraphConditionalHandle cond,
+                                                                  const double *__restrict__ part, int np,
+                                                                  double *__restrict__ scal, double tol, int max_iter,
+                                                                  int *__restrict__ it, double *__restrict__ rr_hist)
+{
+    grid_dependency_wait();
+    __shared__ double sred[kDotThreads / 32];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+    if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    double rr = 0.0;
+    for (int w = 0; w < kDotThreads / 32; ++w) rr += sred[w];
+    scal[S_RR] = rr;
+    const int k = ++*it;
+    rr_hist[k] = rr;
+    const double rel = sqrt(fmax(0.0, rr) / scal[S_BB]);
+    cudaGraphSetConditional(cond, (k < max_iter && !(rel <= tol)) ? 1u : 0u);
+}
+
+// One PCG iteration after the first (q = A p ... p = z + beta p); loop: the
+// while node's condition when this is the body of the loop graph.
+int pcg_iteration(amgt_amg *h, double *x, cudaStream_t s, const cudaGraphConditionalHandle *loop = nullptr)
 {
     Level &v0 = h->lv[0];
     if (h->prm.packed) AMGT_TRY(pbsr_dot(&v0.pA, h->p, h->q, h->part, h->grid0, s));
@@ -861,31 +897,24 @@ int pcg_iteration(amgt_amg *h, double *x, cudaStream_t s)
         AMGT_TRY(sell_dot(v0.sA, mode, h->p, h->q, h->part, s, h->sm_count));
     else AMGT_TRY(spmv_dot(AMGT_DOUBLE, &v0.A, h->p, h->q, h->part, h->grid0, s));
     AMGT_LAUNCH_PDL(reduce_kernel, 1, kDotThreads, 0, s, h->part, h->grid0, h->scal, (int)S_PQ, (int)OP_ALPHA);
-    AMGT_LAUNCH_PDL(axpy2_dot_kernel, kDotGrid, kDotThreads, 0, s, h->n0, h->scal, h->p, h->q, x, h->r, h->part);
-    AMGT_LAUNCH_PDL(reduce_kernel, 1, kDotThreads, 0, s, h->part, kDotGrid, h->scal, (int)S_RR, (int)OP_STORE);
-    AMGT_CUDA_TRY(cudaMemcpyAsync(h->pinned, h->scal + S_RR, sizeof(double), cudaMemcpyDeviceToHost, s));
+    const bool sweep = h->lv.size() > 1;  // level 0 smooths: its first sweep comes with the new residual
+    AMGT_LAUNCH_PDL(axpy2_dot_kernel, kDotGrid, kDotThreads, 0, s, h->n0, h->scal, h->p, h->q, x, h->r, h->part,
+                    (const double *)v0.inv_l1, h->prm.relax_weight, sweep ? v0.u : (double *)nullptr);
+    if (loop) {
+        AMGT_LAUNCH_PDL(pcg_continue_kernel, 1, kDotThreads, 0, s, *loop, (const double *)h->part, kDotGrid, h->scal,
+                        h->prm.tol, h->prm.max_iter, h->loop_it, h->loop_rr);
+    } else {
+        AMGT_LAUNCH_PDL(reduce_kernel, 1, kDotThreads, 0, s, h->part, kDotGrid, h->scal, (int)S_RR, (int)OP_STORE);
+        AMGT_CUDA_TRY(cudaMemcpyAsync(h->pinned, h->scal + S_RR, sizeof(double), cudaMemcpyDeviceToHost, s));
+    }
     if (h->prm.flexible) AMGT_TRY(dot(h, h->z, h->r, S_ZRPREV, OP_STORE, s));
-    AMGT_TRY(cycle(h, h->r, h->z, s));
+    AMGT_TRY(cycle(h, h->r, h->z, s, sweep));
     AMGT_TRY(dot(h, h->r, h->z, S_RZ, h->prm.flexible ? OP_BETA_FLEX : OP_BETA, s));
     AMGT_LAUNCH_PDL(xpby_kernel, grid_n(h, h->n0), 256, 0, s, h->n0, h->z, h->scal, h->p);
     return AMGT_OK;
 }
 
-// End of a loop iteration inside the loop graph: counts it, keeps ||r||^2
-// and sets the while condition with the host loop's test (relative
-// residual above tol and fewer than max_iter iterations).
-__global__ void pcg_continue_kernel(cudaGraphConditionalHandle cond, const double *__restrict__ scal, double tol,
-                                    int max_iter, int *__restrict__ it, double *__restrict__ rr_hist)
-{
-    const int k = ++*it;
-    const double rr = scal[S_RR];
-    rr_hist[k] = rr;
-    const double rel = sqrt(fmax(0.0, rr) / scal[S_BB]);
-    cudaGraphSetConditional(cond, (k < max_iter && !(rel <= tol)) ? 1u : 0u);
-}
-
-// Builds h->loop: a while node whose body is one PCG iteration plus
-// pcg_continue_kernel.  Returns an error (and the caller keeps the
+// Builds h->loop: a while node whose body is one PCG iteration.  Returns an error (and the caller keeps the
 // one-graph-per-iteration loop) if the runtime does not take it.
 int build_loop_graph(amgt_amg *h, double *x)
 {
@@ -918,14 +947,8 @@ int build_loop_graph(amgt_amg *h, double *x)
     }
     if (e == cudaSuccess) {
         const uint64_t c0 = amgt_kernel_launch_count();
-        rc = pcg_iteration(h, x, h->graph_stream);
-        if (rc == AMGT_OK) {
-            count_launch();
-            h->loop_launches = amgt_kernel_launch_count() - c0;
-            pcg_continue_kernel<<<1, 1, 0, h->graph_stream>>>(cond, h->scal, h->prm.tol, h->prm.max_iter, h->loop_it,
-                                                              h->loop_rr);
-            e = cudaGetLastError();
-        }
+        rc = pcg_iteration(h, x, h->graph_stream, &cond);
+        h->loop_launches = amgt_kernel_launch_count() - c0;
         cudaGraph_t captured = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(h->graph_stream, &captured);
         if (e == cudaSuccess) e = ee;
@@ -976,7 +999,8 @@ int gm_iteration(amgt_amg *h, cudaStream_t s, int use_cond, cudaGraphConditional
 {
     const int m = h->prm.restart;
     const long long n = h->n0;
-    AMGT_TRY(cycle(h, h->gm_vin, h->gm_zout, s));
+    const bool sweep = h->lv.size() > 1;
+    AMGT_TRY(cycle(h, h->gm_vin, h->gm_zout, s, sweep));
     AMGT_LAUNCH_PDL(gm_store_z_kernel, grid_n(h, n), 256, 0, s, n, (const double *)h->gm_zout, (const int *)h->gm_j,
                     h->gmZ);
     AMGT_TRY(op_spmv(h->prm.inner_prec0, 1.0, &h->lv[0].A, h->lv[0].sA, h->gm_zout, 0.0, h->gm_w, s, h->sm_count));
@@ -989,7 +1013,8 @@ int gm_iteration(amgt_amg *h, cudaStream_t s, int use_cond, cudaGraphConditional
     AMGT_LAUNCH_PDL(gm_givens_kernel, 1, kDotThreads, 0, s, cond, use_cond, (const double *)h->gm_part, kDotGrid,
                     h->gm_j, m, h->gm, h->prm.inner_tol, h->loop_it, h->prm.max_iter, h->loop_rr);
     AMGT_LAUNCH_PDL(gm_scale_kernel, grid_n(h, n), 256, 0, s, n, (const double *)h->gm_w, (const int *)h->gm_j, m,
-                    (const double *)h->gm, h->gmV, h->gm_vin);
+                    (const double *)h->gm, h->gmV, h->gm_vin, (const double *)h->lv[0].inv_l1, h->prm.relax_weight,
+                    sweep ? h->lv[0].u : (double *)nullptr);
     return AMGT_OK;
 }
 
@@ -1072,7 +1097,8 @@ int fgmres_ir_solve(amgt_amg *h, const double *b, double *x, int *iterations, do
         // inner solve of A d = r; x += d
         AMGT_LAUNCH(gm_start_kernel, 1, 1, 0, s, m, (const double *)h->scal, (int)S_RR, h->gm, h->gm_j);
         AMGT_LAUNCH(gm_scale_first_kernel, grid_n(h, n), 256, 0, s, n, (const double *)h->r, m,
-                    (const double *)h->gm, h->gmV, h->gm_vin);
+                    (const double *)h->gm, h->gmV, h->gm_vin, (const double *)v0.inv_l1, h->prm.relax_weight,
+                    h->lv.size() > 1 ? v0.u : (double *)nullptr);
         bool done = false;
         if (h->prm.use_graph && !h->gm_loop_failed) {
             const int lrc = build_gm_loop(h);
@@ -1126,7 +1152,10 @@ int amgt::op_residual(int prec, const amgt_bsr *A, const SellMat &S, const doubl
     return spmv_residual(prec, A, f, u, r, s, sm_count);
 }
 
-int amgt::amg_cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s) { return cycle(h, rhs0, out0, s); }
+int amgt::amg_cycle(amgt_amg *h, const double *rhs0, double *out0, bool have_u, cudaStream_t s)
+{
+    return cycle(h, rhs0, out0, s, have_u);
+}
 
 extern "C" {
 

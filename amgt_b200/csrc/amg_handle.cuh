@@ -81,8 +81,9 @@ int op_spmv(int prec, double alpha, const amgt_bsr *A, const SellMat &S, const d
             cudaStream_t s, int sm_count);
 int op_residual(int prec, const amgt_bsr *A, const SellMat &S, const double *f, const double *u, double *r,
                 cudaStream_t s, int sm_count);
-// z = M r: one V(1,1) cycle of h's hierarchy (amg.cu)
-int amg_cycle(amgt_amg *h, const double *rhs0, double *out0, cudaStream_t s);
+// z = M r: one V(1,1) cycle of h's hierarchy; have_u: level 0's first sweep
+// is in lv[0].u already (amg.cu)
+int amg_cycle(amgt_amg *h, const double *rhs0, double *out0, bool have_u, cudaStream_t s);
 // amgt_amg_setup with the coarsest operator inverted per diagonal block:
 // block s has sys_rows[s][L - 1] rows, L the levels set up (nullptr: one
 // block).

@@ -125,13 +125,16 @@ __global__ void b_reduce_kernel(int nsys, const int *__restrict__ sys_tile, cons
     }
 }
 
-// x += alpha_s p; r -= alpha_s q; partial r . r per tile
+// x += alpha_s p; r -= alpha_s q; partial r . r per tile; with u, the cycle's
+// first sweep from a zero guess on the new r
 __global__ void __launch_bounds__(kBThreads) b_axpy2_dot_kernel(int ntiles, int nsys, const int *__restrict__ tile_beg,
                                                                const int *__restrict__ tile_sys,
                                                                const double *__restrict__ scal,
                                                                const double *__restrict__ p,
                                                                const double *__restrict__ q, double *__restrict__ x,
-                                                               double *__restrict__ r, double *__restrict__ part)
+                                                               double *__restrict__ r, double *__restrict__ part,
+                                                               const double *__restrict__ inv_l1, double w,
+                                                               double *__restrict__ u)
 {
     grid_dependency_wait();
     __shared__ double sred[kBThreads / 32];
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(kBThreads) b_axpy2_dot_kernel(int ntiles, int 
             const double ri = r[i] - alpha * q[i];
             r[i] = ri;
             s += ri * ri;
+            if (u) u[i] = w * ri * inv_l1[i];
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
@@ -221,15 +225,16 @@ int b_iteration(amgt_amg *h, Batch *b, double *x, cudaStream_t s, int use_cond, 
 {
     Level &v0 = h->lv[0];
     const int grid = std::min(b->ntiles, 8 * h->sm_count);
+    const bool sweep = h->lv.size() > 1;
     AMGT_TRY(op_spmv(AMGT_DOUBLE, 1.0, &v0.A, v0.sA, h->p, 0.0, h->q, s, h->sm_count));
     AMGT_TRY(dot_b(h, b, h->p, h->q, BS_PQ, BOP_ALPHA, s));
     AMGT_LAUNCH_PDL(b_axpy2_dot_kernel, grid, kBThreads, 0, s, b->ntiles, b->nsys, (const int *)b->tile_beg,
                     (const int *)b->tile_sys, (const double *)b->scal, (const double *)h->p, (const double *)h->q, x,
-                    h->r, b->part);
+                    h->r, b->part, (const double *)v0.inv_l1, h->prm.relax_weight, sweep ? v0.u : (double *)nullptr);
     AMGT_LAUNCH_PDL(b_reduce_kernel, grid_for(8, b->nsys, h->sm_count, 4), 256, 0, s, b->nsys,
                     (const int *)b->sys_tile, (const double *)b->part, b->scal, (int)BS_RR, (int)BOP_RR_TEST,
                     h->prm.tol);
-    AMGT_TRY(amg_cycle(h, h->r, h->z, s));
+    AMGT_TRY(amg_cycle(h, h->r, h->z, sweep, s));
     AMGT_TRY(dot_b(h, b, h->r, h->z, BS_RZ, BOP_BETA, s));
     AMGT_LAUNCH_PDL(b_xpby_kernel, grid, kBThreads, 0, s, b->ntiles, b->nsys, (const int *)b->tile_beg,
                     (const int *)b->tile_sys, (const double *)b->scal, (const double *)h->z, h->p);
@@ -431,7 +436,7 @@ int amgt_amg_solve_batch(amgt_amg *h, const double *bvec, double *x, int *iterat
     AMGT_TRY(op_residual(AMGT_DOUBLE, &v0.A, v0.sA, bvec, x, h->r, s, h->sm_count));
     AMGT_TRY(dot_b(h, b, bvec, bvec, BS_BB, BOP_STORE, s));
     AMGT_TRY(dot_b(h, b, h->r, h->r, BS_RR, BOP_RR_TEST, s));
-    AMGT_TRY(amg_cycle(h, h->r, h->z, s));
+    AMGT_TRY(amg_cycle(h, h->r, h->z, false, s));
     AMGT_TRY(dot_b(h, b, h->r, h->z, BS_RZ, BOP_STORE, s));
     AMGT_CUDA_TRY(cudaMemcpyAsync(h->p, h->z, sizeof(double) * h->n0, cudaMemcpyDeviceToDevice, s));
     bool graph = false;
