@@ -79,15 +79,15 @@ class CSRMatrix:
 
     @property
     def i(self) -> torch.Tensor:
-        return view(self.s.csr.i, self.num_rows + 1, torch.int32)
+        return view(self.s.csr.i, self.num_rows + 1, torch.int32, self)
 
     @property
     def j(self) -> torch.Tensor:
-        return view(self.s.csr.j, self.num_nonzeros, torch.int32)
+        return view(self.s.csr.j, self.num_nonzeros, torch.int32, self)
 
     @property
     def data(self) -> torch.Tensor:
-        return view(self.s.csr.data, self.num_nonzeros, torch.float64)
+        return view(self.s.csr.data, self.num_nonzeros, torch.float64, self)
 
     @property
     def bsr(self):

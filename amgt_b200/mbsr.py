@@ -23,20 +23,23 @@ def _stream(stream=None) -> int:
 
 
 class _DevArray:
-    """__cuda_array_interface__ adapter for a raw device pointer."""
+    """__cuda_array_interface__ adapter for a raw device pointer; a tensor
+    made from it holds it, and so the owner of the memory."""
 
-    def __init__(self, ptr: int, shape, typestr: str):
+    def __init__(self, ptr: int, shape, typestr: str, owner=None):
+        self._owner = owner
         self.__cuda_array_interface__ = {"shape": tuple(shape), "typestr": typestr, "data": (int(ptr), False),
                                          "version": 3, "strides": None}
 
 
-def view(ptr, n: int, dtype: torch.dtype) -> torch.Tensor:
-    """Zero-copy torch view of n elements at a library-owned device pointer."""
+def view(ptr, n: int, dtype: torch.dtype, owner=None) -> torch.Tensor:
+    """Zero-copy torch view of n elements at a library-owned device pointer;
+    `owner`, the object whose collection frees it, lives as long as the view."""
     typestr = {torch.int32: "<i4", torch.float64: "<f8", torch.float32: "<f4", torch.int16: "<i2",
                torch.uint16: "<u2"}[dtype]
     if not ptr or n == 0:
         return torch.empty(0, dtype=dtype, device="cuda")
-    return torch.as_tensor(_DevArray(ptr, (n,), typestr), device="cuda")
+    return torch.as_tensor(_DevArray(ptr, (n,), typestr, owner), device="cuda")
 
 
 def csr_struct(m: int, n: int, ia: torch.Tensor, ja: torch.Tensor, a: torch.Tensor) -> AmgtCsr:
@@ -83,23 +86,23 @@ class Bsr:
         return self.s.blc_num
 
     def ptr(self) -> torch.Tensor:
-        return view(self.s.blcPtr, self.s.blc_row + 1, torch.int32)
+        return view(self.s.blcPtr, self.s.blc_row + 1, torch.int32, self)
 
     def idx(self) -> torch.Tensor:
-        return view(self.s.blcIdx, self.s.blc_num, torch.int32)
+        return view(self.s.blcIdx, self.s.blc_num, torch.int32, self)
 
     def val(self) -> torch.Tensor:
-        return view(self.s.blcVal, 16 * self.s.blc_num, torch.float64)
+        return view(self.s.blcVal, 16 * self.s.blc_num, torch.float64, self)
 
     def map(self) -> torch.Tensor:
-        return view(self.s.blcMap, self.s.blc_num, torch.int16)
+        return view(self.s.blcMap, self.s.blc_num, torch.int16, self)
 
     def shadow(self, prec: int) -> torch.Tensor:
         n = 16 * self.s.blc_num
         if prec == FLOAT:
-            return view(self.s.blcVal_fp32, n, torch.float32)
+            return view(self.s.blcVal_fp32, n, torch.float32, self)
         p = self.s.blcVal_fp16 if prec == HALF else self.s.blcVal_bf16
-        return view(p, n, torch.int16)
+        return view(p, n, torch.int16, self)
 
     def host(self) -> dict:
         """Copies of the arrays on the host (numpy), for checking."""
@@ -269,15 +272,15 @@ class CsrOwned:
 
     @property
     def ia(self) -> torch.Tensor:
-        return view(self.s.i, self.s.num_rows + 1, torch.int32)
+        return view(self.s.i, self.s.num_rows + 1, torch.int32, self)
 
     @property
     def ja(self) -> torch.Tensor:
-        return view(self.s.j, self.s.num_nonzeros, torch.int32)
+        return view(self.s.j, self.s.num_nonzeros, torch.int32, self)
 
     @property
     def a(self) -> torch.Tensor:
-        return view(self.s.data, self.s.num_nonzeros, torch.float64)
+        return view(self.s.data, self.s.num_nonzeros, torch.float64, self)
 
     def free(self, stream=None):
         if self._live:
