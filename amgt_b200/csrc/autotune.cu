@@ -119,9 +119,13 @@ int amgt_spmm_rm(int prec, int engine, double alpha, const amgt_bsr *A, int nvec
     cudaStream_t s = (cudaStream_t)stream;
     if (A->blc_num == 0 || A->col == 0) return scale_vector((long long)A->row * nvec, beta, Y, st->sm_count, s);
     if (!X || !A->blcPtr || !A->blcIdx) return AMGT_ERR_INVALID;
-    // AUTO without a measured choice: the CUDA-core form, faster than the
-    // tensor-core one at every size measured (spmm_tc.cu)
-    int kind = engine == AMGT_ENGINE_TENSOR_CORE ? 1 : 0, wpc = 8;
+    // AUTO without a measured choice: the CUDA-core form (32 right-hand
+    // sides: 7-point 64^3 49 us against 76 on the tensor cores, 27-point 31 to
+    // 42 against 68 to 82; 8: 17 against 37), but for odd counts above 8 on
+    // rows of few blocks, whose scalar accesses then dominate (27: 7-point 88
+    // against 69; 27-point, 24 blocks a row: 55 against 73)
+    const bool scalar = nvec % 2 != 0 && nvec > 8 && (long long)A->blc_num < 12LL * A->blc_row;
+    int kind = engine == AMGT_ENGINE_TENSOR_CORE || (engine == AMGT_ENGINE_AUTO && scalar) ? 1 : 0, wpc = 8;
     if (engine == AMGT_ENGINE_AUTO) {
         Choice c;
         if (lookup(A, prec, nvec, &c)) {

@@ -235,9 +235,10 @@ AMGT_API int amgt_spmm(int prec, double alpha, const amgt_bsr *A, int nvec,
  * into tf32 high and low parts so that the products carry fp32 accuracy;
  * the result is combined with beta * Y in fp64 (so Y = B, alpha = -1,
  * beta = 1 gives an fp64 residual of products computed on the tensor
- * cores).  prec DOUBLE: fp64 on the CUDA cores.  engine CUDA_CORE: a warp
- * per block row, a lane per right-hand side.  engine AUTO: amgt_autotune's
- * choice for (A, prec, nvec), else the CUDA cores.
+ * cores).  prec DOUBLE: fp64 on the CUDA cores.  engine CUDA_CORE: 4 to 16
+ * lanes per block row, two right-hand sides each.  engine AUTO: amgt_autotune's
+ * choice for (A, prec, nvec), else the CUDA cores (the tensor cores for odd
+ * nvec > 8 on matrices of fewer than 12 blocks per block row).
  * An fp32 request on a matrix whose exact fp16 shadow holds every value
  * reads that shadow.  Never blocks the host. */
 #define AMGT_ENGINE_AUTO 0
