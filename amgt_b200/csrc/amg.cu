@@ -1567,6 +1567,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
     {
         const int64_t *hf = nullptr;
         if ((rc = read_back(xflags + 3 * num_interp + 2, 1, s, &hf))) goto fail;
+        if ((rc = check_device_error(s))) goto fail;
         if (hf[0] != 0) {
             rc = AMGT_ERR_INVALID;  // singular coarsest operator
             goto fail;

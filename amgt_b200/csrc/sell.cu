@@ -45,7 +45,10 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
         const bool on = s < d.nslices;
         const int b = s * (8 >> lt) + lane / gl;
         const int k0 = on && b < d.brow ? d.ptr[b] : 0, k1 = on && b < d.brow ? d.ptr[b + 1] : 0;
-        int cnt01 = 0, cnt23 = 0, lo = 0x7FFFFFFF, hi = -1;
+        // entries of two scalar rows in the halves of one word (at most 65,532
+        // each: sell_wanted); unsigned, the upper half uses its top bit
+        uint32_t cnt01 = 0, cnt23 = 0;
+        int lo = 0x7FFFFFFF, hi = -1;
 #pragma unroll 4
         for (int k = k0 + lane % gl; k < k1; k += gl) {
             const uint32_t mp = d.map[k];
@@ -61,8 +64,8 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
             cnt01 += __shfl_xor_sync(FULL, cnt01, o);
             cnt23 += __shfl_xor_sync(FULL, cnt23, o);
         }
-        int len = max(max(cnt01 & 0xFFFF, cnt01 >> 16), max(cnt23 & 0xFFFF, cnt23 >> 16));
-        len = __reduce_max_sync(FULL, len);
+        const int len = (int)__reduce_max_sync(FULL, max(max(cnt01 & 0xFFFFu, cnt01 >> 16),
+                                                         max(cnt23 & 0xFFFFu, cnt23 >> 16)));
         lo = __reduce_min_sync(FULL, lo);
         hi = __reduce_max_sync(FULL, hi);
         const int w = max(1, (len + (1 << lt) - 1) >> lt);  // the product reads a slice's first step
@@ -92,13 +95,15 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
 // block row read the same block; the lanes of a warp write the same step of
 // neighbouring rows), its blocks in order, kFillU blocks' columns, bitmaps
 // and first values in flight.  The rest of the slice is cleared (column base,
-// value zero).  with_idx: write the columns too.
+// value zero).  with_idx: write the columns too.  A row that the size pass
+// found shorter than it is raises the error word and writes nothing beyond
+// its slice.
 constexpr int kFillU = 4;
 
 template <typename V>
 __global__ void __launch_bounds__(kSellThreads) sell_fill_kernel(const __grid_constant__ SellDesc d,
                                                                 const V *__restrict__ src, V *__restrict__ dst,
-                                                                int with_idx)
+                                                                int with_idx, int *__restrict__ err)
 {
     const int lt = d.log_t, tm = (1 << lt) - 1;
     for (int row = blockIdx.x * kSellThreads + threadIdx.x; row < ((d.m + 31) & ~31); row += gridDim.x * kSellThreads) {
@@ -115,10 +120,12 @@ __global__ void __launch_bounds__(kSellThreads) sell_fill_kernel(const __grid_co
         V *vr = dst + row0;
         int j = 0;
         auto put = [&](int col, V v) {
-            const int e = 32 * (j >> lt) + (j & tm);
-            if (i16) i16[e] = (unsigned short)(col - cb);
-            else if (i32) i32[e] = col;
-            vr[e] = v;
+            if (j < w) {
+                const int e = 32 * (j >> lt) + (j & tm);
+                if (i16) i16[e] = (unsigned short)(col - cb);
+                else if (i32) i32[e] = col;
+                vr[e] = v;
+            }
             ++j;
         };
         const V *sq = src + 4 * q;
@@ -149,6 +156,7 @@ __global__ void __launch_bounds__(kSellThreads) sell_fill_kernel(const __grid_co
                 }
             }
         }
+        if (j > w) raise_error(err, DEV_ERR_CAPACITY);
         while (j < w) put(cb, (V)0);
     }
 }
@@ -414,6 +422,8 @@ int sell_measure(const std::vector<SellJob> &jobs, int64_t *meas, cudaStream_t s
 
 int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaStream_t s, int sm_count)
 {
+    DeviceState *st;
+    AMGT_TRY(device_state(&st));
     for (size_t j = 0; j < jobs.size(); ++j) {
         SellMat &S = *jobs[j].out;
         const long long steps = meas_host[2 * j];
@@ -440,19 +450,19 @@ int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaSt
         int with_idx = 1;  // the first storage type's pass writes the columns
         if (S.val[0]) {
             AMGT_LAUNCH(sell_fill_kernel<double>, grid, kSellThreads, 0, s, d, (const double *)A->blcVal,
-                        (double *)S.val[0], with_idx);
+                        (double *)S.val[0], with_idx, st->err);
             with_idx = 0;
         }
         if (S.val[1]) {
             AMGT_LAUNCH(sell_fill_kernel<float>, grid, kSellThreads, 0, s, d, (const float *)A->blcVal_fp32,
-                        (float *)S.val[1], with_idx);
+                        (float *)S.val[1], with_idx, st->err);
             with_idx = 0;
         }
         for (int k = 2; k < 4; ++k)
             if (S.val[k]) {
                 AMGT_LAUNCH(sell_fill_kernel<unsigned short>, grid, kSellThreads, 0, s, d,
                             (const unsigned short *)(k == 2 ? A->blcVal_fp16 : A->blcVal_bf16),
-                            (unsigned short *)S.val[k], with_idx);
+                            (unsigned short *)S.val[k], with_idx, st->err);
                 with_idx = 0;
             }
     }

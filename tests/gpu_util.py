@@ -41,3 +41,52 @@ def random_csr(orc, m, n, row_len, seed, dense_rows=()):
     ja = np.array(ja, np.int32)
     a = rng.standard_normal(len(ja))
     return orc.CSR(m, n, np.array(ia, np.int32), ja, a)
+
+
+class AllocLog:
+    """Context in which the library allocates through torch: logs every
+    allocation's bytes (self.sizes, in order) and fails those that
+    fail(bytes, index) asks for.  Blocks are held until the context ends;
+    every library object made inside must be freed inside."""
+
+    def __init__(self, amgt, fail=None):
+        import ctypes
+
+        self._amgt, self._fail, self._held, self.sizes, self.failed = amgt, fail, {}, [], 0
+        alloc_t = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p)
+        free_t = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p)
+        self._cb = alloc_t(self._alloc), free_t(lambda ptr, stream, ctx: None)
+        self._ptr = [ctypes.cast(f, ctypes.c_void_p) for f in self._cb]
+
+    def _alloc(self, nbytes, stream, ctx):
+        i = len(self.sizes)
+        self.sizes.append(nbytes)
+        if self._fail and self._fail(nbytes, i):
+            self.failed += 1
+            return None
+        t = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        self._held[t.data_ptr()] = t
+        return t.data_ptr()
+
+    def __enter__(self):
+        torch.cuda.synchronize()
+        assert self._amgt.lib().amgt_set_allocator(*self._ptr, None) == 0
+        return self
+
+    def __exit__(self, *exc):
+        torch.cuda.synchronize()
+        assert self._amgt.lib().amgt_set_allocator(None, None, None) == 0
+        self._held.clear()
+
+
+def sliced_steps(A):
+    """Steps (of 32 slots) of the sliced copy of an operator with the CSR
+    pattern of A, restated on the host: 32 >> t rows a slice, 1 << t lanes a
+    row, each slice as long as its longest row."""
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    lens, avg, t = np.diff(A.ia), A.ja.size / A.m, 0
+    while t < 3 and (A.m << t) // 32 < 24 * sm and avg >= (4 << t):
+        t += 1
+    rows = 32 >> t
+    lens = np.concatenate([lens, np.zeros(-len(lens) % rows, lens.dtype)]).reshape(-1, rows)
+    return int(np.maximum(1, (lens.max(1) + (1 << t) - 1) >> t).sum())

@@ -20,16 +20,18 @@ def _problem(orc, kind):
         return orc.laplacian(61, 53, 47), orc.geometric_hierarchy(61, 53, 47)
     if kind == "lanes8":  # 24,360 rows of about 24 entries: eight lanes a row
         return orc.varcoef27(30, 29, 28, seed=4), orc.geometric_hierarchy(30, 29, 28)
-    # "long_row": the first unknown coupled to every other one
+    # "long_row_k": unknown k coupled to every other one (55,296 entries in row
+    # k of its block row: more than 15 bits in either half of a packed count)
     import scipy.sparse as sp
 
-    dims = (48, 48, 24)
+    dims, k = (48, 48, 24), int(kind[-1])
     S = orc.laplacian(*dims).to_scipy().tolil()
     n = S.shape[0]
-    S[0, 1:] = -1e-4
-    S[1:, 0] = -1e-4
+    others = np.arange(n) != k
+    S[k, others] = -1e-4
+    S[others, k] = -1e-4
     S = sp.csr_matrix(S)
-    S = S + sp.diags(np.where(np.arange(n) == 0, 1e-4 * n, 1e-4))
+    S = S + sp.diags(np.where(others, 1e-4, 1e-4 * n))
     S = sp.csr_matrix(S)
     S.sort_indices()
     return (orc.CSR(n, n, S.indptr.astype(np.int32), S.indices.astype(np.int32), S.data),
@@ -42,7 +44,7 @@ def _solver(A, Ps, **kw):
     return AmgSolver(to_dev(A), [to_dev(P) for P in Ps], default_params(**kw))
 
 
-@pytest.mark.parametrize("kind", ["idx32", "ragged", "lanes8", "long_row"])
+@pytest.mark.parametrize("kind", ["idx32", "ragged", "lanes8", "long_row_0", "long_row_1", "long_row_3"])
 def test_fp64_solve_matches_the_oracle(amgt, orc, kind):
     A, Ps = _problem(orc, kind)
     b = A.to_scipy() @ orc.rand_uniform(3, A.n)
