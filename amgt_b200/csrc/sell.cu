@@ -31,10 +31,11 @@ struct SellDesc {
     int64_t *meas;
     int m, n, brow, nslices, log_t, idx32;
 };
-// Row lengths -> slice widths, offsets and column bases.  A warp per slice:
-// the slice's block rows (8 >> log_t of them) share the lanes evenly (4 <<
-// log_t lanes each); a lane walks every (4 << log_t)-th block of its row and
-// counts the stored entries of the four scalar rows.
+// Row lengths -> slice widths, offsets, column bases and the mask of rows that
+// have entries.  A warp per slice: the slice's block rows (8 >> log_t of them)
+// share the lanes evenly (4 << log_t lanes each); a lane walks every (4 <<
+// log_t)-th block of its row and counts the stored entries of the four scalar
+// rows.
 __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid_constant__ SellDesc d)
 {
     __shared__ int wsum[kSellThreads / 32], wbase;
@@ -64,6 +65,10 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
             cnt01 += __shfl_xor_sync(FULL, cnt01, o);
             cnt23 += __shfl_xor_sync(FULL, cnt23, o);
         }
+        // rows with entries: bit i for the slice's row i
+        const uint32_t have = ((cnt01 & 0xFFFFu) ? 1u : 0u) | ((cnt01 >> 16) ? 2u : 0u) |
+                              ((cnt23 & 0xFFFFu) ? 4u : 0u) | ((cnt23 >> 16) ? 8u : 0u);
+        const uint32_t rows = __reduce_or_sync(FULL, have << (4 * (lane / gl)));
         const int len = (int)__reduce_max_sync(FULL, max(max(cnt01 & 0xFFFFu, cnt01 >> 16),
                                                          max(cnt23 & 0xFFFFu, cnt23 >> 16)));
         lo = __reduce_min_sync(FULL, lo);
@@ -84,7 +89,7 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
         }
         __syncthreads();
         if (on && lane == 0) {
-            d.hdr[s] = make_int4(wbase + wsum[warp], w, hi < 0 ? 0 : lo, 0);
+            d.hdr[s] = make_int4(wbase + wsum[warp], w, hi < 0 ? 0 : lo, (int)rows);
             if (hi >= 0 && hi - lo > 0xFFFF) atomicMax((unsigned long long *)(d.meas + 1), (unsigned long long)(hi - lo));
         }
         __syncthreads();
@@ -94,10 +99,12 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
 // Entries, for one storage type: a lane per scalar row (the four lanes of a
 // block row read the same block; the lanes of a warp write the same step of
 // neighbouring rows), its blocks in order, kFillU blocks' columns, bitmaps
-// and first values in flight.  The rest of the slice is cleared (column base,
-// value zero).  with_idx: write the columns too.  A row that the size pass
-// found shorter than it is raises the error word and writes nothing beyond
-// its slice.
+// and first values in flight.  The rest of the row is filled with zero values
+// at the row's own last column, so that a product reads no x entry that the row
+// does not multiply anyway (a slice may hold rows of two systems of a batch,
+// and 0 * NaN is NaN); an empty row, which has none, is masked in the product.
+// with_idx: write the columns too.  A row that the size pass found shorter
+// than it is raises the error word and writes nothing beyond its slice.
 constexpr int kFillU = 4;
 
 template <typename V>
@@ -118,8 +125,9 @@ __global__ void __launch_bounds__(kSellThreads) sell_fill_kernel(const __grid_co
         int *i32 = with_idx && d.idx32 ? static_cast<int *>(d.sidx) + row0 : nullptr;
         unsigned short *i16 = with_idx && !d.idx32 ? static_cast<unsigned short *>(d.sidx) + row0 : nullptr;
         V *vr = dst + row0;
-        int j = 0;
+        int j = 0, last = cb;
         auto put = [&](int col, V v) {
+            last = col;
             if (j < w) {
                 const int e = 32 * (j >> lt) + (j & tm);
                 if (i16) i16[e] = (unsigned short)(col - cb);
@@ -157,7 +165,7 @@ __global__ void __launch_bounds__(kSellThreads) sell_fill_kernel(const __grid_co
             }
         }
         if (j > w) raise_error(err, DEV_ERR_CAPACITY);
-        while (j < w) put(cb, (V)0);
+        while (j < w) put(last, (V)0);
     }
 }
 
@@ -293,7 +301,7 @@ sell_kernel(const __grid_constant__ SellArgs a)
         } while (rem > 0);
         for (int o = 1; o < (1 << lt); o <<= 1) sum += __shfl_xor_sync(FULL, sum, o);
         if (mine) {
-            const double ax = (double)sum;
+            const double ax = (h.w >> (lane >> lt)) & 1 ? (double)sum : 0.0;  // an empty row's slots are not its own
             if constexpr (EPI == SEPI_SPMV) {
                 const double t = a.alpha * ax;
                 a.out[row] = a.beta == 0.0 ? t : t + a.beta * fv;

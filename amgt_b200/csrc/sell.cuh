@@ -8,15 +8,15 @@
 namespace amgt {
 
 // An operator of the AMG cycle in slices: a warp's worth of rows (32 >> log_t
-// of them, 1 << log_t lanes each) with only the stored entries, zero-padded
-// to the slice's longest row.  Step k of slice s holds entry
-// (k << log_t) + t of row i at 32 (hdr[s].x + k) + (i << log_t) + t: the
-// column minus hdr[s].z (16 bits) or the column (idx32) and the value, in
-// the storage types that the cycle's precisions read.
+// of them, 1 << log_t lanes each) with only the stored entries, padded to the
+// slice's longest row with zeros at the row's own last column.  Step k of slice
+// s holds entry (k << log_t) + t of row i at 32 (hdr[s].x + k) + (i << log_t) +
+// t: the column minus hdr[s].z (16 bits) or the column (idx32) and the value,
+// in the storage types that the cycle's precisions read.
 struct SellMat {
     int m = 0, n = 0, nslices = 0, log_t = 0;
     bool idx32 = false;
-    int4 *hdr = nullptr;  // device [nslices]: first step, steps, column base
+    int4 *hdr = nullptr;  // device [nslices]: first step, steps, column base, mask of non-empty rows
     void *idx = nullptr;
     void *val[4] = {nullptr, nullptr, nullptr, nullptr};  // fp64, fp32, fp16, bf16
 };
