@@ -281,8 +281,9 @@ spmm_cc_kernel(const __grid_constant__ MvArgs a)
                 }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
+                if (u > 0 && k + u >= k1) break;  // the same for the group; a re-read block's infinity would meet zero x
                 acc_t v[16];
-                block_values<PREC>(a.val, min(k + u, k1 - 1), v);  // past the row's end: zero x
+                block_values<PREC>(a.val, k + u, v);
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
 #pragma unroll

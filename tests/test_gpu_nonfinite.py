@@ -37,3 +37,38 @@ def test_nan_right_hand_side_stays_in_its_system(amgt, orc):
             continue
         sl = slice(s * n, (s + 1) * n)
         assert torch.equal(x0[sl], x1[sl]) and it0[s] == it1[s] and rel0[s] == rel1[s], s
+
+
+@pytest.mark.parametrize("nvec", [1, 7, 8, 16, 24, 32])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_spmm_keeps_a_stored_infinity(amgt, orc, nvec, prec):
+    """Block rows of 1 to 8 blocks whose last block holds an infinity: its
+    row's result is that infinity (x > 0), every other row's is as without
+    it."""
+    import scipy.sparse as sp
+
+    nb = 48
+    rows, cols, vals = [], [], []
+    rng = np.random.default_rng(3)
+    for b in range(nb):
+        k = 1 + b % 8
+        for j in range(k):
+            for r in range(4):
+                rows.append(4 * b + r), cols.append(4 * ((b + 5 * j) % nb) + (r + j) % 4), vals.append(rng.uniform(0.5, 1))
+    S = sp.csr_matrix((vals, (rows, cols)), shape=(4 * nb, 4 * nb))
+    S.sort_indices()
+    A = orc.CSR(4 * nb, 4 * nb, S.indptr.astype(np.int32), S.indices.astype(np.int32), S.data.copy())
+    last = A.ia[1:] - 1  # row r's last entry lies in its block row's last block
+    X = 0.5 + np.ascontiguousarray(np.stack([np.abs(orc.rand_uniform(v, A.n)) for v in range(nvec)], axis=1))
+    hit = np.arange(0, A.m, 4) + np.arange(nb) % 4  # one row per block row
+    a = A.a.copy()
+    a[last[hit]] = np.inf
+    out = []
+    for v in (A.a, a):
+        G = amgt.Bsr.from_csr(*to_dev(orc.CSR(A.m, A.n, A.ia, A.ja, v)))
+        if prec:
+            G.make_shadow(prec)
+        out.append(G.spmm_rm(torch.from_numpy(X).cuda(), prec=prec, engine=1).cpu().numpy())
+    other = np.setdiff1d(np.arange(A.m), hit)
+    assert np.all(out[1][hit] == np.inf)
+    np.testing.assert_array_equal(out[1][other], out[0][other])
