@@ -342,7 +342,7 @@ __device__ int sym_reduce_hashed(int lane, int cnt, unsigned long long *s, int *
 // Upper bound of pairs per A block row (sum of the selected B row
 // lengths); ub[brA] = 0 so that an exclusive scan gives scratch offsets.
 // Also clears the symbolic pass's counters: ccnt[0 .. brA], csrcnt[0 .. m],
-// stats[0 .. 3] and *nmedium.
+// stats[0 .. 4] and *nmedium.
 __global__ void spgemm_ub_kernel(int m, int brA, const int *__restrict__ aptr, const int *__restrict__ aidx,
                                  const int *__restrict__ bptr, int64_t *__restrict__ ub, int *__restrict__ ccnt,
                                  int *__restrict__ csrcnt, int64_t *__restrict__ stats, int *__restrict__ nmedium)
@@ -360,7 +360,7 @@ __global__ void spgemm_ub_kernel(int m, int brA, const int *__restrict__ aptr, c
         for (int q = 0; q < 4; ++q)
             if (4 * b + q <= m) csrcnt[4 * b + q] = 0;
         if (b == 0) {
-            stats[0] = stats[1] = stats[2] = stats[3] = 0;
+            for (int i = 0; i < 5; ++i) stats[i] = 0;
             *nmedium = 0;
         }
     }
@@ -1277,6 +1277,29 @@ __device__ __forceinline__ void row4_global(const typename NumT<PREC>::val_t *__
     }
 }
 
+// *flag = 1 if one of the 16-byte groups of values holds an infinity or NaN.
+// Bound by HBM: the 27-point 72 x 64 x 80 operator's 283 MB.
+template <int PREC>
+__global__ void __launch_bounds__(256) nonfinite_kernel(const uint4 *__restrict__ v, long long n, int *__restrict__ flag)
+{
+    constexpr uint32_t e = PREC == AMGT_DOUBLE ? 0x7FF00000u
+                           : PREC == AMGT_FLOAT ? 0x7F800000u
+                           : PREC == AMGT_HALF ? 0x7C007C00u
+                                               : 0x7F807F80u;  // exponent bits of a 32-bit word
+    auto bad = [](uint32_t w) -> bool {
+        if constexpr (PREC == AMGT_DOUBLE || PREC == AMGT_FLOAT) return (w & e) == e;
+        else return (w & e & 0xFFFFu) == (e & 0xFFFFu) || (w & e & 0xFFFF0000u) == (e & 0xFFFF0000u);
+    };
+    bool any = false;
+#pragma unroll 4
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const uint4 t = __ldg(v + i);
+        any |= bad(t.y) || bad(t.w);
+        if constexpr (PREC != AMGT_DOUBLE) any |= bad(t.x) || bad(t.z);  // fp64: the low words hold no exponent
+    }
+    if (any) *flag = 1;
+}
+
 // A row of the numeric pass, read two rows ahead of its use, and this
 // lane's A block of its first 32 (the range of the B row it selects),
 // read one row ahead.
@@ -1309,11 +1332,11 @@ __device__ __forceinline__ NumRow num_row(int b, int brA, const int *__restrict_
 // sequential addition order without lists, ranks or rounds.  Lane r of a quad
 // computes row r of the product from the stored entries of its row of the A
 // block (an FMA per entry, k ascending: the staged kernel's chain without its
-// zero terms, which change no finite sum; with a non-finite B value an
-// unstored A entry adds no NaN, as in the reference's scalar branch, where
-// the staged kernel computes 0 * Inf), reading B rows straight from L1 / L2;
-// accumulators for up to kNumWideCap C blocks in shared memory, 128 bytes
-// each.  The row's headers are read ahead of their use.
+// zero terms, which change no finite sum), reading B rows straight from L1 /
+// L2; accumulators for up to kNumWideCap C blocks in shared memory, 128 bytes
+// each.  When B holds an infinity or NaN (*nonfinite), the zero terms count:
+// 0 * Inf is NaN in the staged and the gathered kernel, so every entry of A's
+// blocks is taken then, stored or not.  The row's headers are read ahead of their use.
 // 27-point 72 x 64 x 80 squared (5.5e7 pairs, 75 C blocks a row): 2.35 ms
 // against the staged kernel's 4.21 ms with 64 accumulators (longer rows in
 // global memory) and 3.48 ms with 80.  On short B rows the quads idle and the
@@ -1329,12 +1352,13 @@ spgemm_numeric_wide_kernel(int m, int brA, int cap, const int *__restrict__ aptr
                            int *__restrict__ csr_j, double *__restrict__ csr_a, const int64_t *__restrict__ ub_off,
                            const int *__restrict__ skey, const uint16_t *__restrict__ smap,
                            const uint16_t *__restrict__ pslot, unsigned long long *__restrict__ cflags,
-                           void *__restrict__ cextra)
+                           void *__restrict__ cextra, const int *__restrict__ nonfinite)
 {
     bool not32 = false, not16 = false;
     using T = NumT<PREC>;
     using acc_t = typename T::acc_t;
     constexpr int S = 8, U = kNumWideU;
+    const uint32_t unstored = *nonfinite ? 0xFu : 0u;
     extern __shared__ __align__(16) unsigned char num_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, r = lane & 3;
@@ -1422,7 +1446,7 @@ spgemm_numeric_wide_kernel(int m, int brA, int cap, const int *__restrict__ aptr
                 int tc[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) tc[u] = tn[u];
-                const uint32_t nib = (__shfl_sync(FULL, maf, i) >> (4 * r)) & 0xFu;
+                const uint32_t nib = ((__shfl_sync(FULL, maf, i) >> (4 * r)) & 0xFu) | unstored;
                 const typename T::val_t *ap = aval + 16LL * (cur.a0 + ib + i) + 4 * r;
                 if (i + 1 < chunk) {
                     ji = __shfl_sync(FULL, j0f, i + 1);
@@ -1440,7 +1464,7 @@ spgemm_numeric_wide_kernel(int m, int brA, int cap, const int *__restrict__ aptr
                             tc[u] = slot_of(jg < lc, jc + jg, qc + jg);
                         }
                     }
-                    if (nib == 0) continue;  // no stored entry in this lane's row (no warp-wide operation below)
+                    if (nib == 0) continue;  // no entry to take in this lane's row (no warp-wide operation below)
                     acc_t s[U][4], bk[U][4];
                     int kk = __ffs(nib) - 1;
                     acc_t av = T::ld(ap, kk);
@@ -2115,9 +2139,12 @@ template <int PREC>
 static int launch_numeric_wide(const amgt_bsr *A, const void *aval, const amgt_bsr *B, const void *bval, amgt_bsr *C,
                                void *cshadow, amgt_csr *Ccsr, const int64_t *ub_off, const int *skey,
                                const uint16_t *smap, const uint16_t *pslot, cudaStream_t s, int sm_count,
-                               unsigned long long *cflags, void *cextra)
+                               int *nonfinite, unsigned long long *cflags, void *cextra)
 {
     using V = typename NumT<PREC>::val_t;
+    const long long groups = (long long)B->blc_num * (long long)sizeof(V);  // 16 values a block, 16 bytes a group
+    AMGT_LAUNCH(nonfinite_kernel<PREC>, grid_for(1024, groups, sm_count, 8), 256, 0, s, (const uint4 *)bval, groups,
+                nonfinite);
     // accumulators for the longest row, or twice the average one (longer
     // rows accumulate in C)
     const int cap = std::max(32, std::min({C->max_blc_per_row, (int)(2LL * C->blc_num / A->blc_row), kNumWideCap}));
@@ -2129,7 +2156,7 @@ static int launch_numeric_wide(const amgt_bsr *A, const void *aval, const amgt_b
                 smem, s, A->row, A->blc_row, cap, A->blcPtr, A->blcIdx, A->blcMap, (const V *)aval, B->blcPtr,
                 B->blcIdx, (const V *)bval, C->blcPtr, C->blcIdx, C->blcMap, C->blcVal, cshadow,
                 Ccsr ? Ccsr->i : nullptr, Ccsr ? Ccsr->j : nullptr, Ccsr ? Ccsr->data : nullptr, ub_off, skey, smap,
-                pslot, cflags, cextra);
+                pslot, cflags, cextra, (const int *)nonfinite);
     return AMGT_OK;
 }
 
@@ -2140,7 +2167,7 @@ static int launch_numeric_wide(const amgt_bsr *A, const void *aval, const amgt_b
 template <int PREC>
 static int launch_numeric(const amgt_bsr *A, const void *aval, const amgt_bsr *B, const void *bval, amgt_bsr *C,
                           void *cshadow, amgt_csr *Ccsr, const int64_t *ub_off, const int *skey,
-                          const uint16_t *smap, const uint16_t *pslot, cudaStream_t s, int sm_count,
+                          const uint16_t *smap, const uint16_t *pslot, cudaStream_t s, int sm_count, int *nonfinite,
                           unsigned long long *cflags = nullptr, void *cextra = nullptr)
 {
     if (A->blc_row == 0) return AMGT_OK;
@@ -2155,7 +2182,7 @@ static int launch_numeric(const amgt_bsr *A, const void *aval, const amgt_bsr *B
     // level-1 R (A P), the staged one is as fast: 1.11 against 1.12 ms)
     if (C->max_blc_per_row > kNumCapWide && 48LL * A->blc_row < (long long)C->blc_num)
         return launch_numeric_wide<PREC>(A, aval, B, bval, C, cshadow, Ccsr, ub_off, skey, smap, pslot, s, sm_count,
-                                         cflags, cextra);
+                                         nonfinite, cflags, cextra);
     if (C->max_blc_per_row > kNumCap && 24LL * A->blc_row < (long long)C->blc_num)
         return launch_numeric_cap<PREC, kNumCapWide>(A, aval, B, bval, C, cshadow, Ccsr, ub_off, skey, smap, pslot, s,
                                                      sm_count, cflags, cextra);
@@ -2443,27 +2470,27 @@ int spgemm_impl(int prec, const amgt_bsr *A, const amgt_bsr *B, amgt_bsr *C, amg
         if (Ccsr && brA > 0)
             AMGT_LAUNCH(spgemm_csr_kernel, grid_for(kNumWarps, brA, st->sm_count, 8), 32 * kNumWarps, 0, s, m, brA,
                         C->blcPtr, C->blcIdx, C->blcMap, C->blcVal, Ccsr->i, Ccsr->j, Ccsr->data);
-    } else
-    switch (prec) {
-    case AMGT_DOUBLE:
-        rc = launch_numeric<AMGT_DOUBLE>(A, A->blcVal, B, B->blcVal, C, cshadow, Ccsr, ub_off, skey, smap, pslot, s,
-                                         st->sm_count, fuse ? reinterpret_cast<unsigned long long *>(fuse->flags)
-                                                            : nullptr,
-                                         cextra);
-        break;
-    case AMGT_FLOAT:
-        rc = launch_numeric<AMGT_FLOAT>(A, Atmp.blcVal_fp32, B, Btmp.blcVal_fp32, C, cshadow, Ccsr, ub_off, skey,
-                                        smap, pslot, s, st->sm_count,
-                                        fuse ? reinterpret_cast<unsigned long long *>(fuse->flags) : nullptr, cextra);
-        break;
-    case AMGT_HALF:
-        rc = launch_numeric<AMGT_HALF>(A, Atmp.blcVal_fp16, B, Btmp.blcVal_fp16, C, cshadow, Ccsr, ub_off, skey,
-                                       smap, pslot, s, st->sm_count);
-        break;
-    default:
-        rc = launch_numeric<AMGT_BF16>(A, Atmp.blcVal_bf16, B, Btmp.blcVal_bf16, C, cshadow, Ccsr, ub_off, skey,
-                                       smap, pslot, s, st->sm_count);
-        break;
+    } else {
+        int *nonfinite = reinterpret_cast<int *>(&stats[4]);  // cleared by spgemm_ub_kernel
+        unsigned long long *flags = fuse ? reinterpret_cast<unsigned long long *>(fuse->flags) : nullptr;
+        switch (prec) {
+        case AMGT_DOUBLE:
+            rc = launch_numeric<AMGT_DOUBLE>(A, A->blcVal, B, B->blcVal, C, cshadow, Ccsr, ub_off, skey, smap, pslot,
+                                             s, st->sm_count, nonfinite, flags, cextra);
+            break;
+        case AMGT_FLOAT:
+            rc = launch_numeric<AMGT_FLOAT>(A, Atmp.blcVal_fp32, B, Btmp.blcVal_fp32, C, cshadow, Ccsr, ub_off, skey,
+                                            smap, pslot, s, st->sm_count, nonfinite, flags, cextra);
+            break;
+        case AMGT_HALF:
+            rc = launch_numeric<AMGT_HALF>(A, Atmp.blcVal_fp16, B, Btmp.blcVal_fp16, C, cshadow, Ccsr, ub_off, skey,
+                                           smap, pslot, s, st->sm_count, nonfinite);
+            break;
+        default:
+            rc = launch_numeric<AMGT_BF16>(A, Atmp.blcVal_bf16, B, Btmp.blcVal_bf16, C, cshadow, Ccsr, ub_off, skey,
+                                           smap, pslot, s, st->sm_count, nonfinite);
+            break;
+        }
     }
     if (rc) goto fail;
     C->csr_nnz = nnzC;

@@ -72,3 +72,51 @@ def test_spmm_keeps_a_stored_infinity(amgt, orc, nvec, prec):
     other = np.setdiff1d(np.arange(A.m), hit)
     assert np.all(out[1][hit] == np.inf)
     np.testing.assert_array_equal(out[1][other], out[0][other])
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2, 3])
+@pytest.mark.parametrize("kernel", ["staged", "wide"])
+def test_spgemm_nonfinite_entries_meet_unstored_ones(amgt, orc, kernel, prec):
+    """A block product multiplies unstored entries as zeros, so an infinity
+    of B against an unstored entry of A gives NaN, and one of A against an
+    unstored entry of B too, whichever of the staged and the wide-row kernel
+    the sizes pick: the kinds of all C values equal those of dense 4x4 block
+    products (which of them are infinite or NaN does not depend on the order
+    of sums of one sign)."""
+    T = orc.laplacian(64, 32, 20) if kernel == "staged" else orc.box(40, 40, 24)
+    rng = np.random.default_rng(21)
+    a, b = (np.abs(rng.uniform(0.5, 1, T.ja.size)) for _ in range(2))
+    a[rng.integers(0, a.size, 3)] = np.inf
+    b[rng.integers(0, b.size, 5)] = np.inf
+    b[rng.integers(0, b.size, 2)] = np.nan
+    A, B = orc.CSR(T.m, T.n, T.ia, T.ja, a), orc.CSR(T.m, T.n, T.ia, T.ja, b)
+    GA, GB = amgt.Bsr.from_csr(*to_dev(A)), amgt.Bsr.from_csr(*to_dev(B))
+    if prec:
+        GA.make_shadow(prec), GB.make_shadow(prec)
+    GC, csr = amgt.spgemm(GA, GB, prec=prec)
+    c = GC.host()
+    lens = np.diff(c["bptr"])  # enough block rows for these two kernels, and the rule between them
+    assert lens.size >= 64 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert (lens.mean() > 48 and lens.max() > 64) == (kernel == "wide")
+    RA, RB = orc.csr2bsr(A), orc.csr2bsr(B)
+    # only block rows that a non-finite block reaches can hold a non-finite value
+    va, vb = RA.bval.reshape(-1, 4, 4), RB.bval.reshape(-1, 4, 4)
+    brow = np.repeat(np.arange(RA.bptr.size - 1), np.diff(RA.bptr))
+    badb = np.unique(np.repeat(np.arange(RB.bptr.size - 1), np.diff(RB.bptr))[~np.isfinite(vb).all((1, 2))])
+    hit = np.unique(brow[~np.isfinite(va).all((1, 2)) | np.isin(RA.bidx, badb)])
+    got = c["bval"].reshape(-1, 4, 4)
+    finite = np.ones(got.shape[0], bool)
+    for i in hit:
+        C = {}
+        with np.errstate(invalid="ignore"):
+            for p in range(RA.bptr[i], RA.bptr[i + 1]):
+                k = RA.bidx[p]
+                for q in range(RB.bptr[k], RB.bptr[k + 1]):
+                    j = RB.bidx[q]
+                    C[j] = C.get(j, 0.0) + (va[p][:, :, None] * vb[q][None, :, :]).sum(1)
+        for t in range(c["bptr"][i], c["bptr"][i + 1]):
+            finite[t] = False
+            want = C[c["bidx"][t]]
+            np.testing.assert_array_equal(np.isnan(got[t]), np.isnan(want), err_msg=f"block row {i}")
+            np.testing.assert_array_equal(np.isinf(got[t]), np.isinf(want), err_msg=f"block row {i}")
+    assert hit.size > 0 and np.isfinite(got[finite]).all()
