@@ -2149,8 +2149,10 @@ static int launch_numeric_wide(const amgt_bsr *A, const void *aval, const amgt_b
     // rows accumulate in C)
     const int cap = std::max(32, std::min({C->max_blc_per_row, (int)(2LL * C->blc_num / A->blc_row), kNumWideCap}));
     const int smem = kNumWarps * cap * 16 * (int)sizeof(typename NumT<PREC>::acc_t);
+    // always the largest size: the attribute belongs to the function, and
+    // another host thread may launch a smaller or larger product now
     AMGT_CUDA_TRY(cudaFuncSetAttribute(spgemm_numeric_wide_kernel<PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem));
+                                       kNumWarps * kNumWideCap * 16 * (int)sizeof(typename NumT<PREC>::acc_t)));
     const int per_sm = std::max(1, std::min(kNumWideCtas, 227 * 1024 / (smem + 1024)));
     AMGT_LAUNCH(spgemm_numeric_wide_kernel<PREC>, grid_for(kNumWarps, A->blc_row, sm_count, per_sm), 32 * kNumWarps,
                 smem, s, A->row, A->blc_row, cap, A->blcPtr, A->blcIdx, A->blcMap, (const V *)aval, B->blcPtr,
