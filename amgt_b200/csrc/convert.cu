@@ -1177,9 +1177,11 @@ int csr_to_bsr_impl(const amgt_csr *A, amgt_bsr *out, amgt_stream_t stream, int 
         const long long want = 40LL * A->num_nonzeros / m;
         const int cap = (int)std::min<long long>(kFsCapMax, std::max<long long>(kFsCapMin, (want + 15) & ~15LL));
         const int fs_bytes = kFsWarps * cap * kFsEntry;
+        // always the largest size: the attribute belongs to the function, and
+        // another host thread may launch a smaller or larger stage now
         if (fs_bytes > 48 * 1024)
             AMGT_CUDA_TRY(cudaFuncSetAttribute(csr2bsr_fill_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               fs_bytes));
+                                               kFsWarps * kFsCapMax * kFsEntry));
         AMGT_LAUNCH(csr2bsr_fill_sorted_kernel, grid_for(8 * kFsWarps, brow, st->sm_count, 16), 32 * kFsWarps,
                     fs_bytes, s, m, A->i, A->j, A->data, brow, slowf, out->blcPtr, out->blcIdx, out->blcMap,
                     out->blcVal, slotb, fx, cap);

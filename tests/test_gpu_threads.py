@@ -3,7 +3,7 @@ differently."""
 import pytest
 import torch
 
-from gpu_util import to_dev
+from gpu_util import assert_bsr_equal, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,23 @@ def test_host_threads_with_wide_products_of_different_sizes(amgt, orc):
         return run
 
     assert _in_threads([work(i % 2) for i in range(4)]) == []
+
+
+def test_host_threads_converting_long_rows_of_different_lengths(amgt, orc):
+    """Conversions of matrices of 24.4 and 25.4 entries a row, whose fill
+    passes stage different amounts of shared memory (both above 48 KB):
+    threads converting both at once all succeed, bit for bit."""
+    mats = [orc.box(20, 20, 20), orc.box(40, 40, 24)]
+    want = [orc.csr2bsr(A) for A in mats]
+    devs = [to_dev(A) for A in mats]
+    torch.cuda.synchronize()
+
+    def work(k):
+        def run(st):
+            for _ in range(1500):
+                G = amgt.Bsr.from_csr(*devs[k], stream=st)
+            assert_bsr_equal(G, want[k])
+
+        return run
+
+    assert _in_threads([work(i % 2) for i in range(8)]) == []
