@@ -1134,7 +1134,32 @@ int fgmres_ir_solve(amgt_amg *h, const double *b, double *x, int *iterations, do
     return AMGT_OK;
 }
 
+// CTAs (partials) of level 0's fused A p . p
+void set_dot_grid(amgt_amg *h)
+{
+    const Level &v0 = h->lv[0];
+    h->grid0 = h->prm.packed ? pbsr_grid(&v0.pA, h->sm_count)
+               : sell_has(v0.sA, storage_mode(&v0.A, AMGT_DOUBLE)) ? sell_dot_grid(v0.sA, h->sm_count)
+                                                                   : epi_grid(&v0.A, h->sm_count);
+}
+
 }  // namespace
+
+void amgt::drop_sliced_copies(amgt_amg *h, cudaStream_t s)
+{
+    for (Level &v : h->lv) {
+        sell_free(v.sA, s);
+        sell_free(v.sP, s);
+        sell_free(v.sR, s);
+    }
+    set_dot_grid(h);
+    // the graphs that read them are captured again by the next solve
+    for (cudaGraphExec_t *g : {&h->graph, &h->loop, &h->gm_loop}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+    if (h->batch) drop_batch_graph(h->batch);
+}
 
 int amgt::op_spmv(int prec, double alpha, const amgt_bsr *A, const SellMat &S, const double *x, double beta,
                   double *y, cudaStream_t s, int sm_count)
@@ -1546,7 +1571,29 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
         if ((rc = alloc_n(&v.u, v.n, s)) || (rc = alloc_n(&v.t, v.n, s))) goto fail;
         if (l > 0 && ((rc = alloc_n(&v.f, v.n, s)) || (rc = alloc_n(&v.s, v.n, s)))) goto fail;
     }
-    // the sliced copies, in the storage types that the cycle's products read
+    // Krylov vectors and scalars
+    h->n0 = h->lv[0].n;
+    h->grid0 = h->prm.packed ? pbsr_grid(&h->lv[0].pA, h->sm_count) : epi_grid(&h->lv[0].A, h->sm_count);
+    if ((rc = alloc_n(&h->r, h->n0, s)) || (rc = alloc_n(&h->z, h->n0, s)) || (rc = alloc_n(&h->p, h->n0, s)) ||
+        (rc = alloc_n(&h->q, h->n0, s)) || (rc = alloc_n(&h->scal, S_NSCAL, s)) ||
+        (rc = alloc_n(&h->part, std::max({h->grid0, sell_dot_grid(h->lv[0].sA, h->sm_count), kDotGrid}), s)) ||
+        (rc = alloc_n(&h->loop_it, 1, s)) ||
+        (rc = alloc_n(&h->loop_rr, (size_t)h->prm.max_iter + 1, s)))
+        goto fail;
+    if (fgm) {
+        const int m = h->prm.restart;
+        if ((rc = alloc_n(&h->gmV, (size_t)(m + 1) * h->n0, s)) || (rc = alloc_n(&h->gmZ, (size_t)m * h->n0, s)) ||
+            (rc = alloc_n(&h->gm, (size_t)GmLayout{m}.size(), s)) || (rc = alloc_n(&h->gm_vin, h->n0, s)) ||
+            (rc = alloc_n(&h->gm_zout, h->n0, s)) || (rc = alloc_n(&h->gm_w, h->n0, s)) ||
+            (rc = alloc_n(&h->gm_part, (size_t)(m + 1) * kDotGrid, s)) || (rc = alloc_n(&h->gm_j, 1, s)))
+            goto fail;
+        if (cudaMemsetAsync(h->gm, 0, sizeof(double) * GmLayout{m}.size(), s) != cudaSuccess) {
+            rc = AMGT_ERR_CUDA;
+            goto fail;
+        }
+    }
+    // the sliced copies, in the storage types that the cycle's products read;
+    // last, so that they take no memory that the handle cannot do without
     for (SellJob &j : sell) {
         for (int l = 0; l < L; ++l) {
             const Level &v = h->lv[l];
@@ -1563,6 +1610,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
         }
     }
     if ((rc = sell_fill(sell, sell_meas.data(), s, h->sm_count))) goto fail;
+    set_dot_grid(h);
     // coarsest: the inverse's singularity mark (one read-back)
     {
         const int64_t *hf = nullptr;
@@ -1573,29 +1621,6 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
             goto fail;
         }
         if (L == 1) h->lv[L - 1].s = nullptr;
-    }
-    // Krylov vectors and scalars
-    h->n0 = h->lv[0].n;
-    h->grid0 = h->prm.packed ? pbsr_grid(&h->lv[0].pA, h->sm_count)
-               : sell_has(h->lv[0].sA, storage_mode(&h->lv[0].A, AMGT_DOUBLE))
-                   ? sell_dot_grid(h->lv[0].sA, h->sm_count)
-                   : epi_grid(&h->lv[0].A, h->sm_count);
-    if ((rc = alloc_n(&h->r, h->n0, s)) || (rc = alloc_n(&h->z, h->n0, s)) || (rc = alloc_n(&h->p, h->n0, s)) ||
-        (rc = alloc_n(&h->q, h->n0, s)) || (rc = alloc_n(&h->scal, S_NSCAL, s)) ||
-        (rc = alloc_n(&h->part, std::max(h->grid0, kDotGrid), s)) || (rc = alloc_n(&h->loop_it, 1, s)) ||
-        (rc = alloc_n(&h->loop_rr, (size_t)h->prm.max_iter + 1, s)))
-        goto fail;
-    if (fgm) {
-        const int m = h->prm.restart;
-        if ((rc = alloc_n(&h->gmV, (size_t)(m + 1) * h->n0, s)) || (rc = alloc_n(&h->gmZ, (size_t)m * h->n0, s)) ||
-            (rc = alloc_n(&h->gm, (size_t)GmLayout{m}.size(), s)) || (rc = alloc_n(&h->gm_vin, h->n0, s)) ||
-            (rc = alloc_n(&h->gm_zout, h->n0, s)) || (rc = alloc_n(&h->gm_w, h->n0, s)) ||
-            (rc = alloc_n(&h->gm_part, (size_t)(m + 1) * kDotGrid, s)) || (rc = alloc_n(&h->gm_j, 1, s)))
-            goto fail;
-        if (cudaMemsetAsync(h->gm, 0, sizeof(double) * GmLayout{m}.size(), s) != cudaSuccess) {
-            rc = AMGT_ERR_CUDA;
-            goto fail;
-        }
     }
     AMGT_CUDA_TRY(cudaMemsetAsync(h->scal, 0, sizeof(double) * S_NSCAL, s));
     // every host read-back slot of the solvers in one pinned block, so that

@@ -17,6 +17,7 @@ struct MultiRhs;  // multi-right-hand-side work vectors (multirhs.cu)
 void free_multi_rhs(MultiRhs *mr, cudaStream_t s);
 struct Batch;     // per-system data of a batch of systems (batch.cu)
 void free_batch(Batch *b, cudaStream_t s);
+void drop_batch_graph(Batch *b);
 
 struct Level {
     amgt_bsr A{}, P{}, R{};
@@ -81,6 +82,9 @@ int op_spmv(int prec, double alpha, const amgt_bsr *A, const SellMat &S, const d
             cudaStream_t s, int sm_count);
 int op_residual(int prec, const amgt_bsr *A, const SellMat &S, const double *f, const double *u, double *r,
                 cudaStream_t s, int sm_count);
+// Frees the sliced copies (optional ones) of a handle between two solves:
+// memory for an allocation that would fail; products go back to the blocks.
+void drop_sliced_copies(amgt_amg *h, cudaStream_t s);
 // z = M r: one V(1,1) cycle of h's hierarchy; have_u: level 0's first sweep
 // is in lv[0].u already (amg.cu)
 int amg_cycle(amgt_amg *h, const double *rhs0, double *out0, bool have_u, cudaStream_t s);

@@ -206,6 +206,12 @@ void free_batch(Batch *b, cudaStream_t s)
     delete b;
 }
 
+void drop_batch_graph(Batch *b)
+{
+    if (b->loop) cudaGraphExecDestroy(b->loop);
+    b->loop = nullptr;
+}
+
 }  // namespace amgt
 
 using namespace amgt;

@@ -433,11 +433,20 @@ extern "C" int amgt_amg_solve_multi(amgt_amg *h, int nrhs, const double *B, doub
     if (!h || nrhs < 1 || nrhs > 32 || !B || !X) return AMGT_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
     MultiRhs *mr = nullptr;
-    AMGT_TRY(make_multi_rhs(h, nrhs, s, &mr));
     Level &v0 = h->lv[0];
-    // level 0 inside the correction reads inner_prec0's values
-    if (!(h->prm.inner_prec0 == AMGT_FLOAT && v0.A.exact_prec == AMGT_HALF && v0.A.blcVal_fp16))
-        AMGT_TRY(amgt_bsr_make_shadow(&v0.A, h->prm.inner_prec0, stream));
+    auto prepare = [&]() -> int {
+        AMGT_TRY(make_multi_rhs(h, nrhs, s, &mr));
+        // level 0 inside the correction reads inner_prec0's values
+        if (!(h->prm.inner_prec0 == AMGT_FLOAT && v0.A.exact_prec == AMGT_HALF && v0.A.blcVal_fp16))
+            AMGT_TRY(amgt_bsr_make_shadow(&v0.A, h->prm.inner_prec0, stream));
+        return AMGT_OK;
+    };
+    int prc = prepare();
+    if (prc == AMGT_ERR_ALLOC) {  // the sliced copies, which only the other solves read, make room
+        drop_sliced_copies(h, s);
+        prc = prepare();
+    }
+    AMGT_TRY(prc);
     const long long n = h->n0, cnt_all = n * nrhs;
     const int nv = nrhs;
     AMGT_CUDA_TRY(cudaMemsetAsync(mr->cnt, 0, sizeof(int) * 40, s));

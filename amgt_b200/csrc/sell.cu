@@ -420,7 +420,7 @@ int sell_measure(const std::vector<SellJob> &jobs, int64_t *meas, cudaStream_t s
         S.log_t = pick_log_t(jobs[j].A, sm_count);
         const int rows = 32 >> S.log_t;
         S.nslices = (S.m + rows - 1) / rows;
-        AMGT_TRY(alloc_n(&S.hdr, (size_t)S.nslices, s));
+        if (alloc_n(&S.hdr, (size_t)S.nslices, s)) continue;  // no memory: no copy
         SellDesc d = describe(jobs[j]);
         d.meas = meas + 2 * j;
         AMGT_LAUNCH(sell_measure_kernel, grid_for(kSellThreads / 32, S.nslices, sm_count, 8), kSellThreads, 0, s, d);
@@ -434,6 +434,7 @@ int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaSt
     AMGT_TRY(device_state(&st));
     for (size_t j = 0; j < jobs.size(); ++j) {
         SellMat &S = *jobs[j].out;
+        if (!S.hdr) continue;
         const long long steps = meas_host[2 * j];
         // a few long rows among short ones: the padding would outweigh the
         // dense blocks' zeros (and 32 steps is the unit of 32-bit offsets)
@@ -444,14 +445,18 @@ int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaSt
         S.idx32 = meas_host[2 * j + 1] > 0xFFFF;
         const size_t ne = (size_t)(32 * steps);
         unsigned char *p = nullptr;
-        AMGT_TRY(alloc_n(&p, ne * (S.idx32 ? 4 : 2), s));
+        int rc = alloc_n(&p, ne * (S.idx32 ? 4 : 2), s);
         S.idx = p;
         const int bytes[4] = {8, 4, 2, 2};
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < 4 && !rc; ++k)
             if (jobs[j].storages & (1u << k)) {
-                AMGT_TRY(alloc_n(&p, ne * bytes[k], s));
+                rc = alloc_n(&p, ne * bytes[k], s);
                 S.val[k] = p;
             }
+        if (rc) {  // no memory: the products stay on the blocks
+            sell_free(S, s);
+            continue;
+        }
         const SellDesc d = describe(jobs[j]);
         const int grid = grid_for(kSellThreads, S.m, sm_count, 16);
         const amgt_bsr *A = jobs[j].A;

@@ -38,8 +38,8 @@ bool sell_wanted(const amgt_bsr *A);
 // measure launches the pass that sizes the slices, writing per job the
 // total steps and the widest column span to meas[2 j], meas[2 j + 1]
 // (device, zeroed by the caller); fill allocates and fills the copies with
-// those numbers on the host.  A copy whose padding would be too large is
-// left out (out->hdr is null).
+// those numbers on the host.  A copy whose padding would be too large, or for
+// which the allocator has no memory, is left out (out->hdr is null).
 int sell_measure(const std::vector<SellJob> &jobs, int64_t *meas, cudaStream_t s, int sm_count);
 int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaStream_t s, int sm_count);
 void sell_free(SellMat &S, cudaStream_t s);

@@ -46,7 +46,7 @@ def random_csr(orc, m, n, row_len, seed, dense_rows=()):
 class AllocLog:
     """Context in which the library allocates through torch: logs every
     allocation's bytes (self.sizes, in order) and fails those that
-    fail(bytes, index) asks for.  Blocks are held until the context ends;
+    fail(sizes so far, this one last) asks for.  Blocks are held until the context ends;
     every library object made inside must be freed inside."""
 
     def __init__(self, amgt, fail=None):
@@ -59,9 +59,8 @@ class AllocLog:
         self._ptr = [ctypes.cast(f, ctypes.c_void_p) for f in self._cb]
 
     def _alloc(self, nbytes, stream, ctx):
-        i = len(self.sizes)
         self.sizes.append(nbytes)
-        if self._fail and self._fail(nbytes, i):
+        if self._fail and self._fail(self.sizes):
             self.failed += 1
             return None
         t = torch.empty(nbytes, dtype=torch.uint8, device="cuda")

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import to_dev
+from gpu_util import AllocLog, sliced_steps, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -78,3 +78,45 @@ def test_reduced_levels_and_transfers_converge_fp64_verified(amgt, orc, prec):
     r = b - A.to_scipy() @ x.cpu().numpy()
     assert np.linalg.norm(r) <= 1.0000001e-8 * np.linalg.norm(b)
     assert it < 60
+
+
+def _solve_all(amgt, A, Ps, b, fail=None, multi=False):
+    """Setup, solve (and a solve of two right-hand sides, and another solve)
+    under the logging allocator."""
+    amgt.set_level_policy([0])
+    try:
+        with AllocLog(amgt, fail) as log:
+            S = _solver(A, Ps, exact_storage=0)
+            out = [S.solve(b)]
+            if multi:
+                X, its, rel = S.solve_multi(torch.stack([b, b], 1).contiguous())
+                out += [(X[:, 1].contiguous(), its[1], rel[1]), S.solve(b)]
+            S.free()
+    finally:
+        amgt.set_level_policy([])
+    return log, out
+
+
+@pytest.mark.parametrize("what", ["header", "columns", "values", "multi"])
+def test_no_memory_for_a_copy_keeps_the_blocks(amgt, orc, what):
+    """The copies are optional: when the allocator has no memory for a part
+    of A_0's (its slice headers, columns or values), the setup goes on
+    and the products run on the blocks; when it has none for the vectors of
+    a multi-right-hand-side solve while copies are held, they are given back
+    and the solve goes on.  Same iterations and solutions to 1e-9."""
+    dims = (60, 58, 56)
+    A, Ps = orc.laplacian(*dims), orc.geometric_hierarchy(*dims)
+    b = torch.from_numpy(A.to_scipy() @ orc.rand_uniform(6, A.n)).cuda()
+    # A_0's copy: slices of 32 rows, 16-bit offsets, 8-byte values; its headers
+    # are the first ones made
+    hdr, columns, values = 16 * -(-A.m // 32), 2 * 32 * sliced_steps(A), 8 * 32 * sliced_steps(A)
+    log, ref = _solve_all(amgt, A, Ps, b, multi=what == "multi")
+    assert log.sizes.count(columns) == log.sizes.count(values) == 1
+    fail = {"header": lambda s: s[-1] == hdr and s.count(hdr) == 1, "columns": lambda s: s[-1] == columns,
+            "values": lambda s: s[-1] == values,
+            "multi": lambda s: s[-1] == 8 * 2 * A.n and s.count(8 * 2 * A.n) == 1}[what]  # the first multivector
+    log, out = _solve_all(amgt, A, Ps, b, fail, what == "multi")
+    assert log.failed == 1
+    for (x, it, rel), (x0, it0, _) in zip(out, ref):
+        assert it == it0 and rel <= 1e-8
+        assert torch.linalg.norm(x - x0) <= 1e-9 * torch.linalg.norm(x0)
