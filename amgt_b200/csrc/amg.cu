@@ -1271,7 +1271,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
     bool l1_fused0 = false;  // level 0's l1 norms written by A's conversion
     std::vector<SellJob> sell;         // operators that get a sliced copy, ...
     std::vector<int64_t> sell_meas;    // ... and its size as measured on the device
-    const size_t nflags = fused16.size(), nslots = 3 * nflags;  // exactness flags, then two slots per sliced copy
+    const size_t nflags = fused16.size(), nslots = 4 * nflags;  // exactness flags, then three slots per sliced copy
     pm.mark(-1, s);
     if ((rc = alloc_n(&xflags, nslots, s))) goto fail;
     if (cudaMemsetAsync(xflags, 0, sizeof(int64_t) * nslots, s) != cudaSuccess) {
@@ -1524,7 +1524,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
             rc = bsr_exact_check(mats[i].first, xflags + slot, &o, s, h->sm_count);
             own16[slot] = o;
         }
-        std::vector<int64_t> f(nflags + 2 * sell.size(), 0);
+        std::vector<int64_t> f(nflags + kSellMeas * sell.size(), 0);
         for (size_t i0 = 0; i0 < f.size() && !rc; i0 += 63) {
             const int k = (int)std::min<size_t>(63, f.size() - i0);
             const int64_t *hf = nullptr;
@@ -1539,8 +1539,8 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
         }
         if (rc) goto fail;
     }
-    for (size_t i0 = sell_meas.size(); i0 < 2 * sell.size(); i0 = sell_meas.size()) {  // no flags were read back
-        const int k = (int)std::min<size_t>(63, 2 * sell.size() - i0);
+    for (size_t i0 = sell_meas.size(); i0 < kSellMeas * sell.size(); i0 = sell_meas.size()) {  // no flags were read back
+        const int k = (int)std::min<size_t>(63, kSellMeas * sell.size() - i0);
         const int64_t *hf = nullptr;
         if ((rc = read_back(xflags + nflags + i0, k, s, &hf))) goto fail;
         sell_meas.insert(sell_meas.end(), hf, hf + k);

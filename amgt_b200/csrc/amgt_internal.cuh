@@ -130,6 +130,8 @@ int scale_vector(long long n, double beta, double *y, int sm_count, cudaStream_t
 // Value mode that products of A at `prec` read (an AMGT_* precision or an
 // exact narrow storage mode of spmv_common.cuh).
 int storage_mode(const amgt_bsr *A, int prec);
+// Lanes per block row of the products on A's blocks.
+int spmv_lanes(const amgt_bsr *A);
 
 // Fused SpMV forms (spmv.cu): r = f - A u; u_out = u + w (f - A u) .* inv_l1;
 // out = A u with per-CTA partials of u . out (grid CTAs, from epi_grid);

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
         if (on && lane == 0) {
             d.hdr[s] = make_int4(wbase + wsum[warp], w, hi < 0 ? 0 : lo, (int)rows);
             if (hi >= 0 && hi - lo > 0xFFFF) atomicMax((unsigned long long *)(d.meas + 1), (unsigned long long)(hi - lo));
+            if (w > 64) atomicMax((unsigned long long *)(d.meas + 2), (unsigned long long)w);
         }
         __syncthreads();
     }
@@ -422,10 +423,29 @@ int sell_measure(const std::vector<SellJob> &jobs, int64_t *meas, cudaStream_t s
         S.nslices = (S.m + rows - 1) / rows;
         if (alloc_n(&S.hdr, (size_t)S.nslices, s)) continue;  // no memory: no copy
         SellDesc d = describe(jobs[j]);
-        d.meas = meas + 2 * j;
+        d.meas = meas + kSellMeas * j;
         AMGT_LAUNCH(sell_measure_kernel, grid_for(kSellThreads / 32, S.nslices, sm_count, 8), kSellThreads, 0, s, d);
     }
     return AMGT_OK;
+}
+
+// A long row among short ones is a serial chain on both forms: one warp adds
+// its slice step after step (0.45 us a step beyond a warp's ordinary share
+// where the copy streams from HBM, 0.15 where half of L2 holds it), lpr lanes
+// walk its blocks (2 / lpr us a block).  True when the chain loses more than
+// the smaller copy wins in bytes (5 TB/s, 10 from L2).  Measured, us a
+// product, copy against blocks: 128 x 128 x 64 7-point with four rows of 135
+// entries 70 against 76, of 263 127 against 106, of 1,032 465 against 293
+// (without 23 against 46); its next level with the latter 453 against 190;
+// 64^3 with rows of 263 43 against 73, of 1,030 151 against 259.
+static bool slice_too_long(const SellJob &j, long long steps, long long longest, int sm_count)
+{
+    const int vbytes = (j.storages & 1u) ? 8 : (j.storages & 2u) ? 4 : 2;  // the widest storage read
+    const double bytes = 32.0 * steps * ((j.out->idx32 ? 4 : 2) + vbytes), blocks = (16.0 * vbytes + 6) * j.A->blc_num;
+    const bool l2 = bytes < 64e6;
+    const double share = (double)steps / (8.0 * SellShape<AMGT_DOUBLE, SEPI_RESID>::ctas * sm_count);
+    const double chain = (longest - share) * (l2 ? 0.15 : 0.45) - 2.0 * j.A->max_blc_per_row / spmv_lanes(j.A);
+    return longest > 0 && chain > (blocks - bytes) / (l2 ? 10e6 : 5e6);
 }
 
 int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaStream_t s, int sm_count)
@@ -435,22 +455,24 @@ int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaSt
     for (size_t j = 0; j < jobs.size(); ++j) {
         SellMat &S = *jobs[j].out;
         if (!S.hdr) continue;
-        const long long steps = meas_host[2 * j];
-        // a few long rows among short ones: the padding would outweigh the
-        // dense blocks' zeros (and 32 steps is the unit of 32-bit offsets)
-        if (32LL * steps > 2LL * jobs[j].A->csr_nnz + 65536 || steps > 0x3FFFFFFF) {
+        const long long steps = meas_host[kSellMeas * j], longest = meas_host[kSellMeas * j + 2];
+        S.idx32 = meas_host[kSellMeas * j + 1] > 0xFFFF;
+        // long rows among short ones: the padding would outweigh the dense
+        // blocks' zeros (and 32 steps is the unit of 32-bit offsets), or one
+        // warp would walk a slice for longer than the bytes saved win
+        if (32LL * steps > 2LL * jobs[j].A->csr_nnz + 65536 || steps > 0x3FFFFFFF ||
+            slice_too_long(jobs[j], steps, longest, sm_count)) {
             sell_free(S, s);
             continue;
         }
-        S.idx32 = meas_host[2 * j + 1] > 0xFFFF;
         const size_t ne = (size_t)(32 * steps);
         unsigned char *p = nullptr;
         int rc = alloc_n(&p, ne * (S.idx32 ? 4 : 2), s);
         S.idx = p;
-        const int bytes[4] = {8, 4, 2, 2};
+        const int width[4] = {8, 4, 2, 2};
         for (int k = 0; k < 4 && !rc; ++k)
             if (jobs[j].storages & (1u << k)) {
-                rc = alloc_n(&p, ne * bytes[k], s);
+                rc = alloc_n(&p, ne * width[k], s);
                 S.val[k] = p;
             }
         if (rc) {  // no memory: the products stay on the blocks

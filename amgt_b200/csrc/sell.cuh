@@ -36,10 +36,11 @@ struct SellJob {
 bool sell_wanted(const amgt_bsr *A);
 // Two steps, so that one host read-back (the caller's) sizes every copy:
 // measure launches the pass that sizes the slices, writing per job the
-// total steps and the widest column span to meas[2 j], meas[2 j + 1]
-// (device, zeroed by the caller); fill allocates and fills the copies with
-// those numbers on the host.  A copy whose padding would be too large, or for
+// total steps, the widest column span above 65,535 and the longest slice above
+// 64 steps to meas[kSellMeas j ...] (device, zeroed by the caller); fill allocates and fills the copies with
+// those numbers on the host.  A copy that would not pay (see there), or for
 // which the allocator has no memory, is left out (out->hdr is null).
+constexpr int kSellMeas = 3;
 int sell_measure(const std::vector<SellJob> &jobs, int64_t *meas, cudaStream_t s, int sm_count);
 int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaStream_t s, int sm_count);
 void sell_free(SellMat &S, cudaStream_t s);

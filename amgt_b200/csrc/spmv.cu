@@ -409,6 +409,8 @@ static int pick_lpr(const amgt_bsr *A, int mode)
     return 32;
 }
 
+int spmv_lanes(const amgt_bsr *A) { return pick_lpr(A, AMGT_DOUBLE); }
+
 // Lanes a row is given when it runs: 2-byte values move few bytes per
 // lane, so with the 8-lane segment layout half the lanes (each group
 // holding two of its segments, same sums) keep more rows in flight

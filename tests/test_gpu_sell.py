@@ -2,8 +2,9 @@
 that uses them: fp64 solves take the oracle's iterations with x within 1e-9
 of its (the bars of the block path, test_gpu_amg.py), on shapes that reach
 each form: 16-bit offsets, 32-bit columns (a slice's columns spread over more
-than 65,535), several lanes per row, ragged sizes, operators that get no copy
-because one long row would pad its slice, and reduced-precision storage."""
+than 65,535), several lanes per row, ragged sizes, one long row, operators
+that get no copy because long rows would pad their slices or one warp would
+walk too long a slice, and reduced-precision storage."""
 import numpy as np
 import pytest
 import torch
@@ -78,6 +79,54 @@ def test_reduced_levels_and_transfers_converge_fp64_verified(amgt, orc, prec):
     r = b - A.to_scipy() @ x.cpu().numpy()
     assert np.linalg.norm(r) <= 1.0000001e-8 * np.linalg.norm(b)
     assert it < 60
+
+
+def _coupled(orc, dims, rows, reach, count, seed=9):
+    """7-point operator with `count` random couplings of each of `rows` to
+    unknowns at most `reach` away (symmetric, diagonally dominant)."""
+    import scipy.sparse as sp
+
+    S = orc.laplacian(*dims).to_scipy()
+    n, rng = S.shape[0], np.random.default_rng(seed)
+    r = np.repeat(rows, count)
+    c = np.concatenate([max(0, min(k - reach, n - 2 * reach - 1)) + rng.choice(2 * reach, count, replace=False)
+                        for k in rows])
+    E = sp.csr_matrix((np.full(r.size, 1e-3), (r, c)), shape=(n, n))
+    E = E + E.T
+    E.setdiag(0)
+    S = sp.csr_matrix(S - E + sp.diags(np.asarray(E.sum(1)).ravel()))
+    S.sort_indices()
+    return orc.CSR(n, n, S.indptr.astype(np.int32), S.indices.astype(np.int32), S.data)
+
+
+@pytest.mark.parametrize("kind", ["padding", "one_slice"])
+def test_operators_that_get_no_copy(amgt, orc, kind):
+    """One row of 60 entries in every slice (padded to seven times the
+    entries), or one slice of 1,000 steps in an operator of 75 MB: no slice
+    columns are allocated for level 0, and the solve converges as the block
+    path does (fp64 residual)."""
+    from amgt_b200.amg import AmgSolver, default_params
+
+    dims = (61, 53, 47) if kind == "padding" else (128, 128, 64)
+    n = int(np.prod(dims))
+    rows = np.arange(5, n, 32) if kind == "padding" else np.array([n // 2])
+    A = _coupled(orc, dims, rows, 3000, 60 if kind == "padding" else 1000)
+    Ps = orc.geometric_hierarchy(*dims)
+    b = A.to_scipy() @ orc.rand_uniform(6, A.n)
+    steps = sliced_steps(A)
+    assert (32 * steps > 2 * A.ja.size + 65536) == (kind == "padding")
+    for M, copied in ((A, False), (orc.laplacian(*dims), True)):
+        amgt.set_level_policy([0])
+        try:
+            with AllocLog(amgt) as log:
+                S = AmgSolver(to_dev(M), [to_dev(P) for P in Ps], default_params(exact_storage=0))
+                if not copied:
+                    x, it, rel = S.solve(torch.from_numpy(b).cuda())
+                S.free()
+        finally:
+            amgt.set_level_policy([])
+        assert log.sizes.count(2 * 32 * sliced_steps(M)) == int(copied)
+    assert np.linalg.norm(b - A.to_scipy() @ x.cpu().numpy()) <= 1.0000001e-8 * np.linalg.norm(b)
 
 
 def _solve_all(amgt, A, Ps, b, fail=None, multi=False):
