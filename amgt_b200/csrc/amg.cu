@@ -1271,7 +1271,7 @@ int amgt::amg_setup_blocks(const amgt_csr *A, int num_interp, const amgt_csr *P,
     bool l1_fused0 = false;  // level 0's l1 norms written by A's conversion
     std::vector<SellJob> sell;         // operators that get a sliced copy, ...
     std::vector<int64_t> sell_meas;    // ... and its size as measured on the device
-    const size_t nflags = fused16.size(), nslots = 4 * nflags;  // exactness flags, then three slots per sliced copy
+    const size_t nflags = fused16.size(), nslots = (1 + kSellMeas) * nflags;  // exactness flags, then each sliced copy's slots
     pm.mark(-1, s);
     if ((rc = alloc_n(&xflags, nslots, s))) goto fail;
     if (cudaMemsetAsync(xflags, 0, sizeof(int64_t) * nslots, s) != cudaSuccess) {

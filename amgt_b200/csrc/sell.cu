@@ -91,6 +91,8 @@ __global__ void __launch_bounds__(kSellThreads) sell_measure_kernel(const __grid
         if (on && lane == 0) {
             d.hdr[s] = make_int4(wbase + wsum[warp], w, hi < 0 ? 0 : lo, (int)rows);
             if (hi >= 0 && hi - lo > 0xFFFF) atomicMax((unsigned long long *)(d.meas + 1), (unsigned long long)(hi - lo));
+            const int last = min(d.m - s * (32 >> lt), 32 >> lt);  // the slice's rows
+            if (rows != (last < 32 ? (1u << last) - 1u : FULL)) d.meas[3] = 1;
             if (w > 64) atomicMax((unsigned long long *)(d.meas + 2), (unsigned long long)w);
         }
         __syncthreads();
@@ -231,13 +233,16 @@ struct SellShape {
 // again instead of predicating each step off (the predicated form compiled to
 // about 340 instructions a slice of seven steps and 36 us a level-0 residual).
 // One wave of CTAs, so that every warp walks several slices.
+// HOLES (the operator has rows without entries) masks their sums by the bits
+// in the slice's header; done for every operator it cost the batch's solve
+// 1.3 % (9.43 against 9.54 ms).
 //
 // Bound by HBM bytes: an entry is 2 + {8, 4, 2} bytes, each vector 8 bytes a
 // row.  128^3 7-point, fp64 from exact fp16 storage, residual: 109 MB in 28
 // us (3.9 TB/s; the block kernel: 183 MB in 41 us); BoomerAMG's level 1 (1.05
 // M rows, 17.6 M entries, 8-byte values): 202 MB in 38 us (5.3 TB/s) against
 // 93 us on 593 MB of blocks.
-template <int MODE, bool IDX32, int EPI>
+template <int MODE, bool IDX32, int EPI, bool HOLES>
 __global__ void __launch_bounds__(kSellThreads, SellShape<MODE, EPI>::ctas)
 sell_kernel(const __grid_constant__ SellArgs a)
 {
@@ -302,7 +307,8 @@ sell_kernel(const __grid_constant__ SellArgs a)
         } while (rem > 0);
         for (int o = 1; o < (1 << lt); o <<= 1) sum += __shfl_xor_sync(FULL, sum, o);
         if (mine) {
-            const double ax = (h.w >> (lane >> lt)) & 1 ? (double)sum : 0.0;  // an empty row's slots are not its own
+            double ax = (double)sum;
+            if constexpr (HOLES) ax = (h.w >> (lane >> lt)) & 1 ? ax : 0.0;  // an empty row's slots are not its own
             if constexpr (EPI == SEPI_SPMV) {
                 const double t = a.alpha * ax;
                 a.out[row] = a.beta == 0.0 ? t : t + a.beta * fv;
@@ -347,8 +353,10 @@ static int launch_sell(const SellMat &S, int mode, SellArgs a, cudaStream_t s, i
 #define AMGT_SELL_CASE(M)                                                                              \
     case M: {                                                                                          \
         const int grid = grid_for(kSellThreads / 32, S.nslices, sm_count, SellShape<M, EPI>::ctas);    \
-        if (S.idx32) AMGT_LAUNCH_PDL((sell_kernel<M, true, EPI>), grid, kSellThreads, 0, s, a);          \
-        else AMGT_LAUNCH_PDL((sell_kernel<M, false, EPI>), grid, kSellThreads, 0, s, a);                 \
+        if (S.idx32 && S.holes) AMGT_LAUNCH_PDL((sell_kernel<M, true, EPI, true>), grid, kSellThreads, 0, s, a); \
+        else if (S.idx32) AMGT_LAUNCH_PDL((sell_kernel<M, true, EPI, false>), grid, kSellThreads, 0, s, a);      \
+        else if (S.holes) AMGT_LAUNCH_PDL((sell_kernel<M, false, EPI, true>), grid, kSellThreads, 0, s, a);      \
+        else AMGT_LAUNCH_PDL((sell_kernel<M, false, EPI, false>), grid, kSellThreads, 0, s, a);                  \
         return AMGT_OK;                                                                                \
     }
     switch (mode) {
@@ -457,6 +465,7 @@ int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaSt
         if (!S.hdr) continue;
         const long long steps = meas_host[kSellMeas * j], longest = meas_host[kSellMeas * j + 2];
         S.idx32 = meas_host[kSellMeas * j + 1] > 0xFFFF;
+        S.holes = meas_host[kSellMeas * j + 3] != 0;
         // long rows among short ones: the padding would outweigh the dense
         // blocks' zeros (and 32 steps is the unit of 32-bit offsets), or one
         // warp would walk a slice for longer than the bytes saved win

@@ -15,7 +15,7 @@ namespace amgt {
 // in the storage types that the cycle's precisions read.
 struct SellMat {
     int m = 0, n = 0, nslices = 0, log_t = 0;
-    bool idx32 = false;
+    bool idx32 = false, holes = false;  // holes: some row has no entry
     int4 *hdr = nullptr;  // device [nslices]: first step, steps, column base, mask of non-empty rows
     void *idx = nullptr;
     void *val[4] = {nullptr, nullptr, nullptr, nullptr};  // fp64, fp32, fp16, bf16
@@ -36,11 +36,12 @@ struct SellJob {
 bool sell_wanted(const amgt_bsr *A);
 // Two steps, so that one host read-back (the caller's) sizes every copy:
 // measure launches the pass that sizes the slices, writing per job the
-// total steps, the widest column span above 65,535 and the longest slice above
-// 64 steps to meas[kSellMeas j ...] (device, zeroed by the caller); fill allocates and fills the copies with
+// total steps, the widest column span above 65,535, the longest slice above 64
+// steps and whether a row is empty to meas[kSellMeas j ...] (device, zeroed by
+// the caller); fill allocates and fills the copies with
 // those numbers on the host.  A copy that would not pay (see there), or for
 // which the allocator has no memory, is left out (out->hdr is null).
-constexpr int kSellMeas = 3;
+constexpr int kSellMeas = 4;
 int sell_measure(const std::vector<SellJob> &jobs, int64_t *meas, cudaStream_t s, int sm_count);
 int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaStream_t s, int sm_count);
 void sell_free(SellMat &S, cudaStream_t s);

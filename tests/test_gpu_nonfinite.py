@@ -8,22 +8,29 @@ from gpu_util import to_dev
 pytestmark = pytest.mark.gpu
 
 
-def test_nan_right_hand_side_stays_in_its_system(amgt, orc):
-    """45 systems of 40 x 35 unknowns and one coarse level: system and coarse
-    sizes (1,400 and 360) are multiples of 4, so no block holds two systems,
-    but not of 16, so slices of the sliced copies (16 or 32 rows) do.  A NaN in one system's
-    right-hand side (whose last slice holds rows of the next one) changes no
-    bit of the others' solutions."""
+@pytest.mark.parametrize("holes", [False, True])
+def test_nan_right_hand_side_stays_in_its_system(amgt, orc, holes):
+    """62 systems of 56 x 37 unknowns and two coarse levels: all sizes (2,072,
+    532, 140) are multiples of 4, so no block holds two systems, but not of
+    32, so slices of the sliced copies do.  A NaN in one system's right-hand
+    side (whose last slice holds rows of the next one) changes no bit of the
+    others' solutions; also with empty rows in the interpolation."""
     from amgt_b200.amg import BatchSolver, default_params
 
-    ns, bad = 45, 40
-    A, P = orc.laplacian(40, 35, 1), orc.geometric_hierarchy(40, 35, 1)[0]
-    n = A.n
+    ns, bad = 62, 40
+    A, Ps = orc.laplacian(56, 37, 1), orc.geometric_hierarchy(56, 37, 1)[:2]
+    n, P = A.n, Ps[0]
+    if holes:  # unknowns 0 .. 7 and 9 are not interpolated
+        keep = np.ones(n, bool)
+        keep[[0, 1, 2, 3, 4, 5, 6, 7, 9]] = False
+        lens = np.where(keep, np.diff(P.ia), 0)
+        sel = np.repeat(keep, np.diff(P.ia))
+        Ps[0] = orc.CSR(P.m, P.n, np.concatenate([[0], np.cumsum(lens)]).astype(np.int32), P.ja[sel], P.a[sel])
     amgt.set_level_policy([0])
     try:
-        S = BatchSolver([(to_dev(A), [to_dev(P)])] * ns, default_params(max_coarse_rows=16384))
-        lv = S.level(0)
-        assert lv["blocks"] >= 65536 and n % 4 == 0 and n % 16 != 0 and P.n % 4 == 0
+        S = BatchSolver([(to_dev(A), [to_dev(P) for P in Ps])] * ns, default_params(max_coarse_rows=16384))
+        assert ns * orc.csr2bsr(Ps[0]).nblk >= 65536  # A_0 and P_0 are copied
+        assert n % 32 != 0 and all(k % 4 == 0 for k in (n, Ps[0].n, Ps[1].n))
         b = torch.from_numpy(orc.rand_uniform(5, ns * n)).cuda()
         x0, it0, rel0, _ = S.solve_batch(b)
         b[bad * n + 7] = float("nan")
