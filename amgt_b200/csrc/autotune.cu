@@ -119,13 +119,12 @@ int amgt_spmm_rm(int prec, int engine, double alpha, const amgt_bsr *A, int nvec
     cudaStream_t s = (cudaStream_t)stream;
     if (A->blc_num == 0 || A->col == 0) return scale_vector((long long)A->row * nvec, beta, Y, st->sm_count, s);
     if (!X || !A->blcPtr || !A->blcIdx) return AMGT_ERR_INVALID;
-    // AUTO without a measured choice: the CUDA-core form (32 right-hand
-    // sides: 7-point 64^3 49 us against 76 on the tensor cores, 27-point 31 to
-    // 42 against 68 to 82; 8: 17 against 37), but for odd counts above 8 on
-    // rows of few blocks, whose scalar accesses then dominate (27: 7-point 88
-    // against 69; 27-point, 24 blocks a row: 55 against 73)
-    const bool scalar = nvec % 2 != 0 && nvec > 8 && (long long)A->blc_num < 12LL * A->blc_row;
-    int kind = engine == AMGT_ENGINE_TENSOR_CORE || (engine == AMGT_ENGINE_AUTO && scalar) ? 1 : 0, wpc = 8;
+    // AUTO without a measured choice: the CUDA-core form, the faster one at
+    // every size and count measured (fp16 storage, us against the tensor cores:
+    // 7-point 64^3, 32 right-hand sides 45.5 / 76.5, 27 52.5 / 69.0, 13 27.0 /
+    // 37.4, 8 12.7 / 36.6; 1,024 block rows, 27 3.4 / 6.0; 27-point 10^3, 27 5.1
+    // / 14.2; 4,921 block rows, 13 8.2 / 14.0)
+    int kind = engine == AMGT_ENGINE_TENSOR_CORE ? 1 : 0, wpc = 8;
     if (engine == AMGT_ENGINE_AUTO) {
         Choice c;
         if (lookup(A, prec, nvec, &c)) {

@@ -17,6 +17,7 @@ enum {
 };
 struct MvArgs {
     int m, n, brow, nvec;
+    int split;  // parts of a block row
     const int *ptr, *idx;
     const uint16_t *map;
     const void *val;

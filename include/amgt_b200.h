@@ -236,9 +236,9 @@ AMGT_API int amgt_spmm(int prec, double alpha, const amgt_bsr *A, int nvec,
  * the result is combined with beta * Y in fp64 (so Y = B, alpha = -1,
  * beta = 1 gives an fp64 residual of products computed on the tensor
  * cores).  prec DOUBLE: fp64 on the CUDA cores.  engine CUDA_CORE: 4 to 16
- * lanes per block row, two right-hand sides each.  engine AUTO: amgt_autotune's
- * choice for (A, prec, nvec), else the CUDA cores (the tensor cores for odd
- * nvec > 8 on matrices of fewer than 12 blocks per block row).
+ * lanes per block row, two right-hand sides each (several such groups per
+ * block row on matrices of few of them).  engine AUTO: amgt_autotune's choice
+ * for (A, prec, nvec), else the CUDA cores.
  * An fp32 request on a matrix whose exact fp16 shadow holds every value
  * reads that shadow.  Never blocks the host. */
 #define AMGT_ENGINE_AUTO 0

@@ -65,3 +65,31 @@ def test_spmm_without_bitmaps_and_misaligned(amgt, orc, nvec, prec):
     for v in range(nvec):
         want = orc.spmv(R, X[:, v], prec=prec)
         assert np.all(np.abs(got[:, v] - want) <= (1e-12 if prec == 0 else 1e-5) * orc.spmv_bound(R, X[:, v], None) + 1e-300)
+
+
+@pytest.mark.parametrize("nvec", [1, 2, 5, 8, 13, 16, 17, 24, 31, 32])
+@pytest.mark.parametrize("dims,pts", [((5, 3, 1), 7), ((19, 11, 9), 27), ((47, 31, 29), 7), ((55, 53, 54), 7)])
+def test_spmm_cuda_core_forms(amgt, orc, dims, pts, nvec):
+    """The CUDA-core form where its lanes per block row, its parts of a block
+    row (8, 4, 2, 1 from 4 to 40,000 block rows) and its access widths change,
+    at fp64, fp32 and fp16 values, beta 0 and not: per row 1e-12 (fp64) or
+    1e-5 (fp32 sums of about 27 terms) of |A||x| + |y|."""
+    T = orc.laplacian(*dims) if pts == 7 else orc.box(*dims)
+    A = orc.CSR(T.m, T.n, T.ia, T.ja, np.random.default_rng(2).uniform(-1, 1, T.ja.size))
+    G = amgt.Bsr.from_csr(*to_dev(A))
+    X = np.ascontiguousarray(np.stack([orc.rand_uniform(v, A.n) for v in range(nvec)], axis=1))
+    Y0 = np.ascontiguousarray(np.stack([orc.rand_uniform(50 + v, A.m) for v in range(nvec)], axis=1))
+    x = torch.from_numpy(X).cuda()
+    S = A.to_scipy()
+    for prec, beta in ((0, 0.0), (0, -0.5), (1, 0.0), (2, -0.5)):
+        if prec:
+            G.make_shadow(prec)
+        M = S.copy()
+        if prec:
+            M.data = M.data.astype(np.float32 if prec == 1 else np.float16).astype(np.float64)
+        y = torch.from_numpy(Y0).cuda()
+        G.spmm_rm(x, y, alpha=1.5, beta=beta, prec=prec, engine=1)
+        want = 1.5 * (M @ X) + beta * Y0
+        bound = 1.5 * (abs(M) @ np.abs(X)) + np.abs(beta * Y0)
+        err = np.abs(y.cpu().numpy() - want)
+        assert np.all(err <= (1e-12 if prec == 0 else 1e-5) * bound + 1e-300)
