@@ -20,6 +20,18 @@ pytestmark = pytest.mark.gpu
 GOLD = os.path.join(os.path.dirname(__file__), "golden")
 
 
+def _random_values(orc, T, seed):
+    return orc.CSR(T.m, T.n, T.ia, T.ja, np.random.default_rng(seed).uniform(-1, 1, T.ja.size))
+
+
+def _with_rows(orc, T, rows, seed):
+    """T with the four rows of block row b replaced by rows[b], random values."""
+    parts = [rows[r // 4] if r // 4 in rows else T.ja[T.ia[r]:T.ia[r + 1]] for r in range(T.m)]
+    ia = np.concatenate([[0], np.cumsum([len(p) for p in parts])]).astype(np.int32)
+    ja = np.concatenate(parts).astype(np.int32)
+    return _random_values(orc, orc.CSR(T.m, T.n, ia, ja, np.zeros(ja.size)), seed)
+
+
 def _pair(orc, kind):
     if kind == "AP_7pt":
         A = orc.laplacian(22, 18, 14)
@@ -79,11 +91,28 @@ def _pair(orc, kind):
         A2 = orc.bsr2csr(orc.spgemm(orc.csr2bsr(A), orc.csr2bsr(A))[0])
         return A, A2
     if kind == "AA_27pt_wide":
-        # A * A of the 27-point pattern: C rows of 50-75 blocks (64-block
-        # shared accumulators, the longer rows in global memory)
+        # A * A of the 27-point pattern: C rows of 50-75 blocks, the wide-row
+        # numeric with every row's accumulators in shared memory
         T = orc.box(40, 40, 24)
         A = orc.CSR(T.m, T.n, T.ia, T.ja, np.random.default_rng(12).uniform(-1, 1, T.ja.size))
         return A, A
+    if kind == "AA_27pt_wide_long":
+        # the same product with three long block rows in A: 40 A blocks (more
+        # than 32) of 100 C blocks and at most 1,024 pairs; 37 A blocks far apart
+        # (C blocks beyond the 112 accumulated in shared memory, values
+        # accumulated in C); 2,000 A blocks (pairs found by searching the pattern)
+        T = orc.box(40, 40, 24)
+        x, y, z = np.meshgrid(np.arange(40), np.arange(4), [0], indexing="ij")
+        near = np.sort((x + 40 * y + 1600 * z).ravel())
+        far = np.sort(np.concatenate([np.arange(4) + 40 * 7 * k for k in range(36)] + [np.arange(4, 8)]))
+        return _with_rows(orc, T, {0: near, 1: far, 2: np.arange(0, 8000, 4)}, 17), _random_values(orc, T, 18)
+    if kind == "LONG_row_staged64":
+        # C rows of 33-48 blocks on average, one long row beyond 64: the staged
+        # numeric with 64-block accumulators, that row's values in C
+        T = orc.laplacian(48, 40, 40)
+        A = _with_rows(orc, T, {0: np.arange(0, 4000, 2)}, 19)
+        B = _random_values(orc, T, 20)
+        return A, orc.bsr2csr(orc.spgemm(orc.csr2bsr(B), orc.csr2bsr(B))[0])
     if kind == "LONG_row_staged":
         # the 7-point operator with its first four rows made long (every
         # second column of the first 4,000): one block row of > 1024 pairs
@@ -124,7 +153,8 @@ def _pair(orc, kind):
 
 
 KINDS = ["AP_7pt", "AP_varcoef27", "RAP_varcoef27", "AA_varcoef27", "AA_5pt", "AAA_27pt", "AP_7pt_large",
-         "AA_7pt_large", "A2A2_9pt", "AAA_7pt_wide", "AA_27pt_wide", "LONG_row_staged", "A2A3_27pt_long", "WIDE_row"]
+         "AA_7pt_large", "A2A2_9pt", "AAA_7pt_wide", "AA_27pt_wide", "AA_27pt_wide_long", "LONG_row_staged",
+         "LONG_row_staged64", "A2A3_27pt_long", "WIDE_row"]
 
 
 @pytest.mark.parametrize("kind", KINDS)
@@ -271,3 +301,52 @@ def test_two_host_threads_on_one_device(amgt, orc):
     for outs in results:
         for GC in outs:
             assert_bsr_equal(GC, RC)
+
+
+@pytest.mark.parametrize("by_level", [0, 1])
+@pytest.mark.parametrize("dyadic", [False, True])
+def test_wide_galerkin_level_shadows(amgt, orc, dyadic, by_level):
+    """Galerkin levels through the wide-row numeric (the identity as first
+    interpolations of a 125-point operator, so that levels 1 and 2 are level 0's
+    values) used in fp32: level 1, computed in fp64, comes with its fp32 shadow;
+    level 2, computed in fp32 by its finer level's precision, with its fp16
+    candidate; multiples of 1/4 are found exact in fp16, random values are not."""
+    import ctypes
+
+    from amgt_b200.amg import AmgSolver, default_params
+    from amgt_b200.mbsr import view
+
+    dims = (40, 40, 24)
+    T = orc.box(*dims)
+    S = abs(T.to_scipy()) @ abs(T.to_scipy())
+    S.sort_indices()
+    n = T.n
+    rng = np.random.default_rng(22)
+    S.data = -rng.integers(1, 5, S.nnz) / 4.0 if dyadic else -rng.uniform(0.1, 1, S.nnz)
+    S.setdiag(256.0)
+    A = orc.CSR(n, n, S.indptr.astype(np.int32), S.indices.astype(np.int32), S.data)
+    eye = orc.CSR(n, n, np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), np.ones(n))
+    R = orc.csr2bsr(A)
+    assert np.diff(R.bptr).mean() > 48 and np.diff(R.bptr).max() > 64
+    amgt.set_level_policy([0, 1])
+    try:
+        H = AmgSolver(to_dev(A), [to_dev(P) for P in [eye, eye] + orc.geometric_hierarchy(*dims)],
+                      default_params(flexible=1, galerkin_by_level=by_level))
+        b = amgt._lib.AmgtBsr()
+        prec = ctypes.c_int()
+        assert amgt.lib().amgt_amg_level(H.h, 1 + by_level, ctypes.byref(b), ctypes.byref(prec)) == 0
+        assert prec.value == 1
+        val = view(b.blcVal, 16 * b.blc_num, torch.float64).cpu().numpy()
+        want = R.bval.astype(np.float32).astype(np.float64) if by_level else R.bval
+        np.testing.assert_array_equal(val, want)
+        assert b.exact_prec == (2 if dyadic else by_level)  # fp32 products are exact in fp32
+        if b.blcVal_fp32:
+            np.testing.assert_array_equal(view(b.blcVal_fp32, val.size, torch.float32).cpu().numpy(),
+                                          val.astype(np.float32))
+        if dyadic:
+            np.testing.assert_array_equal(view(b.blcVal_fp16, val.size, torch.int16).cpu().numpy().view(np.float16),
+                                          val.astype(np.float16))
+        assert b.blcVal_fp32 or dyadic
+        H.free()
+    finally:
+        amgt.set_level_policy([])
