@@ -52,11 +52,13 @@ def test_fp64_solve_matches_the_oracle(amgt, orc, kind):
     xo, it_o, _, _ = orc.Amg(A, Ps).solve(b)
     amgt.set_level_policy([0])
     try:
-        S = _solver(A, Ps)
-        x, it, rel = S.solve(torch.from_numpy(b).cuda())
-        S.free()
+        with AllocLog(amgt) as log:
+            S = _solver(A, Ps)
+            x, it, rel = S.solve(torch.from_numpy(b).cuda())
+            S.free()
     finally:
         amgt.set_level_policy([])
+    assert (4 if kind == "idx32" else 2) * 32 * sliced_steps(A) in log.sizes  # level 0 is copied
     assert it == it_o and rel <= 1e-8
     assert np.linalg.norm(x.cpu().numpy() - xo) <= 1e-9 * np.linalg.norm(xo)
 
@@ -71,11 +73,14 @@ def test_reduced_levels_and_transfers_converge_fp64_verified(amgt, orc, prec):
     b = A.to_scipy() @ orc.rand_uniform(4, A.n)
     amgt.set_level_policy([0, prec])
     try:
-        S = _solver(A, Ps, flexible=1, smooth_prec0=1)
-        x, it, rel = S.solve(torch.from_numpy(b).cuda())
-        S.free()
+        with AllocLog(amgt) as log:
+            S = _solver(A, Ps, flexible=1, smooth_prec0=1)
+            x, it, rel = S.solve(torch.from_numpy(b).cuda())
+            S.free()
     finally:
         amgt.set_level_policy([])
+    steps = sliced_steps(A)  # level 0's copy: columns, 8-byte and 4-byte values
+    assert all(k * 32 * steps in log.sizes for k in (2, 8, 4))
     r = b - A.to_scipy() @ x.cpu().numpy()
     assert np.linalg.norm(r) <= 1.0000001e-8 * np.linalg.norm(b)
     assert it < 60
