@@ -43,7 +43,9 @@ void count_launch();
 // which hides most of the launch gap between dependent kernels (also inside
 // CUDA graphs, where capture turns it into a programmatic edge).  Every
 // kernel launched this way calls grid_dependency_wait() before it touches
-// memory; without a programmatic dependency the wait returns at once.
+// memory that a kernel of the same solve writes (sell_kernel reads its matrix
+// before: the setup that wrote it has ended with a synchronisation); without
+// a programmatic dependency the wait returns at once.
 #define AMGT_LAUNCH_PDL(kernel, grid, block, smem, strm, ...)                 \
     do {                                                                      \
         amgt::count_launch();                                                 \

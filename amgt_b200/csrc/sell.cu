@@ -258,8 +258,8 @@ sell_kernel(const __grid_constant__ SellArgs a)
     const raw_t *val = static_cast<const raw_t *>(a.val) + lane;
     double dot = 0.0;
     int s = (blockIdx.x * kSellThreads + threadIdx.x) >> 5;
-    // the matrix is older than the previous kernel: its first loads need not
-    // wait for it
+    // the setup that wrote the matrix has ended with a synchronisation: its
+    // first loads need not wait for the kernels before
     const int4 none = make_int4(0, 1, 0, 0);
     int4 h = s < a.nslices ? __ldg(a.hdr + s) : none, hn = s + nw < a.nslices ? __ldg(a.hdr + s + nw) : none;
     int c[U];   // columns of the batch to gather next

@@ -357,7 +357,9 @@ AMGT_API int amgt_spmv_segmented_noalloc(int prec, double alpha, const amgt_bsr 
  * (built on demand), fp32 arithmetic, C values rounded to fp64 and a C
  * shadow of the same precision.  If Ccsr != NULL the CSR form of C
  * (BSR2CSR) is also written, by the numeric pass itself (rows of few C
- * blocks) or by a pass right after it.
+ * blocks) or by a pass right after it.  Entries of a block without a stored
+ * value count as zeros where two blocks are multiplied: an infinity or NaN
+ * against one gives NaN.
  * Host-blocking twice (upper bound and C size). */
 AMGT_API int amgt_spgemm(int prec, const amgt_bsr *A, const amgt_bsr *B, amgt_bsr *C,
                 amgt_csr *Ccsr, amgt_stream_t stream);
@@ -425,7 +427,13 @@ AMGT_API void amgt_amg_default_params(amgt_amg_params *p);
 /* Host-blocking (sizes of every level).  The coarsest operator is inverted
  * on the GPU (Gauss-Jordan, partial pivoting); a singular one returns
  * AMGT_ERR_INVALID.  Rejected with AMGT_ERR_INVALID: max_iter outside
- * 1 .. 1000000, tol negative or NaN, max_coarse_rows outside 1 .. 16384. */
+ * 1 .. 1000000, tol negative or NaN, max_coarse_rows outside 1 .. 16384.
+ * Unless `packed`, the handle also holds copies of its larger operators with
+ * only the stored entries, which amgt_amg_solve and amgt_amg_solve_batch read
+ * (2 bytes an entry, or 4, plus the value in each precision used; amgt_autotune's
+ * choices do not apply to them).  A copy for which the allocator has no memory
+ * is left out, and amgt_amg_solve_multi, which does not read them, frees them
+ * when its own vectors find none. */
 AMGT_API int amgt_amg_setup(const amgt_csr *A, int num_interp, const amgt_csr *P,
                             const amgt_amg_params *params, amgt_amg **out,
                             amgt_stream_t stream);
@@ -458,10 +466,11 @@ AMGT_API int amgt_amg_solve(amgt_amg *amg, const double *b, double *x,
  * Refinement in fp64 (R = B - A X with fp64 values; X += D) around a
  * correction A D = R solved by PCG in lockstep over the columns, each with
  * its own scalars and its own stop (inner_tol * ||R_v||), preconditioned by
- * one V(1,1) cycle whose every operator is one amgt_spmm_rm over all
- * columns at its level's precision (reduced-precision levels on the tensor
- * cores; level 0 inside the correction at inner_prec0).  Each correction is
- * one CUDA graph launch.  Stops when every column reaches tol, or after
+ * one V(1,1) cycle whose every operator is one product over all columns at
+ * its level's precision, on the CUDA cores with the cycle's vector updates
+ * fused into it (amgt_autotune's choices are for amgt_spmm_rm and not used;
+ * level 0 inside the correction at inner_prec0).  Each correction is one CUDA
+ * graph launch.  Stops when every column reaches tol, or after
  * max_iter correction iterations in total, or max_outer refinements.
  * iterations[v]: correction iterations column v took; rel_res[v]: its
  * final ||B_v - A X_v|| / ||B_v|| in fp64 (both arrays may be NULL). */

@@ -1,7 +1,7 @@
 """GPU tests of the batching form.
 
 Many right-hand sides on one hierarchy (amgt_amg_solve_multi, every cycle
-operator one tensor-core SpMM over all columns): each column's residual,
+operator one product over all columns): each column's residual,
 checked in fp64 by the oracle, is <= 1e-8, and each column's x agrees with
 the oracle's fp64 AMG-PCG solution of that right-hand side to 1e-6 relative
 (both stop at 1e-8).
@@ -53,10 +53,10 @@ def test_multi_rhs_small(amgt, orc, policy, inner):
     _multi(amgt, orc, (24, 22, 20), 8, policy, inner)
 
 
-def test_multi_rhs_64cubed_32_rhs_tensor_cores(amgt, orc):
+def test_multi_rhs_64cubed_32_rhs(amgt, orc):
     """C4a: 7-point 64^3, 32 right-hand sides (seeds 0..31), levels 1-2
-    fp32 and >= 3 fp16 on the tensor cores, level 0 inside the correction
-    in fp32, fp64 residuals."""
+    fp32 and >= 3 fp16, level 0 inside the correction in fp32, fp64
+    residuals."""
     its, errs = _multi(amgt, orc, (64, 64, 64), 32, [0, 1, 1, 2], 1)
     print(f"C4a: iterations per column {min(its)}..{max(its)}, max error vs fp64 oracle {max(errs):.2e}")
 
