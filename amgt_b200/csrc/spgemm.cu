@@ -2169,8 +2169,8 @@ static int launch_numeric_wide(const amgt_bsr *A, const void *aval, const amgt_b
 template <int PREC>
 static int launch_numeric(const amgt_bsr *A, const void *aval, const amgt_bsr *B, const void *bval, amgt_bsr *C,
                           void *cshadow, amgt_csr *Ccsr, const int64_t *ub_off, const int *skey,
-                          const uint16_t *smap, const uint16_t *pslot, cudaStream_t s, int sm_count, int *nonfinite,
-                          unsigned long long *cflags = nullptr, void *cextra = nullptr)
+                          const uint16_t *smap, const uint16_t *pslot, cudaStream_t s, int sm_count, int64_t npairs,
+                          int *nonfinite, unsigned long long *cflags = nullptr, void *cextra = nullptr)
 {
     if (A->blc_row == 0) return AMGT_OK;
     if (C->max_blc_per_row <= kNumCapNarrow)
@@ -2180,9 +2180,17 @@ static int launch_numeric(const amgt_bsr *A, const void *aval, const amgt_bsr *B
         return launch_numeric_cap<PREC, kNumCapMid>(A, aval, B, bval, C, cshadow, Ccsr, ub_off, skey, smap, pslot, s,
                                                     sm_count, cflags, cextra);
     // more than 48 C blocks a row on average, some beyond 64: the wide-row
-    // kernel (75 a row: 2.35 ms against 4.21; at 38 a row, 128^3 BoomerAMG's
-    // level-1 R (A P), the staged one is as fast: 1.11 against 1.12 ms)
-    if (C->max_blc_per_row > kNumCapWide && 48LL * A->blc_row < (long long)C->blc_num)
+    // kernel, where its quads have B blocks to take and, in fp64, its shared
+    // accumulators hold (nearly) every row.  us, staged against wide, by C
+    // blocks a row and pairs an A block: fp64 70 of 25 3,780 / 2,370, 103 of 25
+    // 3,890 / 2,560, 70 of 6 1,315 / 1,215, but 83 of 5.7 1,360 / 1,470, 75 of 2.9
+    // 825 / 1,200, 123 of 12 2,630 / 3,170 (accumulated in C); fp32 70 of 25 3,270
+    // / 1,640, 83 of 5.7 1,280 / 930, 140 of 14 2,830 / 2,450, but 75 of 2.9 800 /
+    // 880.  At 38 C blocks a row both are as fast.
+    const bool fp64 = PREC == AMGT_DOUBLE;
+    if (C->max_blc_per_row > kNumCapWide && 48LL * A->blc_row < (long long)C->blc_num &&
+        8 * npairs >= (fp64 ? 47LL : 32LL) * A->blc_num &&
+        (!fp64 || C->max_blc_per_row <= kNumWideCap || (long long)C->blc_num <= 96LL * A->blc_row))
         return launch_numeric_wide<PREC>(A, aval, B, bval, C, cshadow, Ccsr, ub_off, skey, smap, pslot, s, sm_count,
                                          nonfinite, cflags, cextra);
     if (C->max_blc_per_row > kNumCap && 24LL * A->blc_row < (long long)C->blc_num)
@@ -2478,19 +2486,19 @@ int spgemm_impl(int prec, const amgt_bsr *A, const amgt_bsr *B, amgt_bsr *C, amg
         switch (prec) {
         case AMGT_DOUBLE:
             rc = launch_numeric<AMGT_DOUBLE>(A, A->blcVal, B, B->blcVal, C, cshadow, Ccsr, ub_off, skey, smap, pslot,
-                                             s, st->sm_count, nonfinite, flags, cextra);
+                                             s, st->sm_count, npairs, nonfinite, flags, cextra);
             break;
         case AMGT_FLOAT:
             rc = launch_numeric<AMGT_FLOAT>(A, Atmp.blcVal_fp32, B, Btmp.blcVal_fp32, C, cshadow, Ccsr, ub_off, skey,
-                                            smap, pslot, s, st->sm_count, nonfinite, flags, cextra);
+                                            smap, pslot, s, st->sm_count, npairs, nonfinite, flags, cextra);
             break;
         case AMGT_HALF:
             rc = launch_numeric<AMGT_HALF>(A, Atmp.blcVal_fp16, B, Btmp.blcVal_fp16, C, cshadow, Ccsr, ub_off, skey,
-                                           smap, pslot, s, st->sm_count, nonfinite);
+                                           smap, pslot, s, st->sm_count, npairs, nonfinite);
             break;
         default:
             rc = launch_numeric<AMGT_BF16>(A, Atmp.blcVal_bf16, B, Btmp.blcVal_bf16, C, cshadow, Ccsr, ub_off, skey,
-                                           smap, pslot, s, st->sm_count, nonfinite);
+                                           smap, pslot, s, st->sm_count, npairs, nonfinite);
             break;
         }
     }

@@ -106,6 +106,18 @@ def _pair(orc, kind):
         near = np.sort((x + 40 * y + 1600 * z).ravel())
         far = np.sort(np.concatenate([np.arange(4) + 40 * 7 * k for k in range(36)] + [np.arange(4, 8)]))
         return _with_rows(orc, T, {0: near, 1: far, 2: np.arange(0, 8000, 4)}, 17), _random_values(orc, T, 18)
+    if kind in ("A27_short_B_rows", "A27_long_C_rows"):
+        # C rows of about 70 blocks from B rows of 3, and of about 130 blocks: beyond
+        # 64 on average, but not the wide-row kernel's (the latter in fp64)
+        T = orc.box(40, 40, 24)
+        off = [0, -4800, 4800] if kind == "A27_short_B_rows" else list(range(0, 80, 4))
+        r = np.repeat(np.arange(T.n), len(off))
+        c = r + np.tile(off, T.n)
+        ok = (c >= 0) & (c < T.n)
+        ia = np.concatenate([[0], np.cumsum(np.bincount(r[ok], minlength=T.n))]).astype(np.int32)
+        ja = c[ok].reshape(-1).astype(np.int32)
+        ja = ja[np.lexsort((ja, r[ok]))]
+        return _random_values(orc, T, 23), _random_values(orc, orc.CSR(T.n, T.n, ia, ja, np.zeros(ja.size)), 24)
     if kind == "LONG_row_staged64":
         # C rows of 33-48 blocks on average, one long row beyond 64: the staged
         # numeric with 64-block accumulators, that row's values in C
@@ -154,7 +166,7 @@ def _pair(orc, kind):
 
 KINDS = ["AP_7pt", "AP_varcoef27", "RAP_varcoef27", "AA_varcoef27", "AA_5pt", "AAA_27pt", "AP_7pt_large",
          "AA_7pt_large", "A2A2_9pt", "AAA_7pt_wide", "AA_27pt_wide", "AA_27pt_wide_long", "LONG_row_staged",
-         "LONG_row_staged64", "A2A3_27pt_long", "WIDE_row"]
+         "LONG_row_staged64", "A27_short_B_rows", "A27_long_C_rows", "A2A3_27pt_long", "WIDE_row"]
 
 
 @pytest.mark.parametrize("kind", KINDS)
