@@ -184,10 +184,13 @@ csr2bsr_count_sorted_kernel(int m, int n, const int *__restrict__ ia, const int 
 // gives its matching entries the rank, the lowest lane's first one the flag.
 // The columns of a warp's 8 block rows come into shared memory, and their
 // slot bytes leave from it, with coalesced accesses when they fit.
-// 27-point 96^3 (23.3 M entries): 209 us, bound by the merge's instructions;
-// one lane per block row, whose stage holds 1,024 entries of 32 block rows and
-// which reads longer ones entry by entry, took 343.  For short rows the quad
-// idles (7-point 128^3 BoomerAMG setup's conversions: 407 us against 225).
+// 27-point 96^3 (23.3 M entries): 131 us, bound by the merge's instructions (the
+// quads of a warp step together; each for itself, one after the other, took
+// 209); one lane per block row, whose stage holds 1,024 entries of 32 block rows
+// and which reads longer ones entry by entry, 332.  9-point: 110 against 186;
+// rows of random columns, which both give up at the 33rd block column: 52
+// against 55.  For short rows the quad idles (7-point 128^3: 89 with a lane per
+// block row).
 __global__ void __launch_bounds__(32 * kStWarps)
 csr2bsr_count_quad_kernel(int m, int n, const int *__restrict__ ia, const int *__restrict__ ja, int brow,
                             int *__restrict__ cnt, int *__restrict__ slow, int *__restrict__ nslow,
@@ -213,32 +216,34 @@ csr2bsr_count_quad_kernel(int m, int n, const int *__restrict__ ia, const int *_
             for (int e = E0 + lane; e < E1; e += 32) sc[e - E0] = __ldg(ja + e);
         __syncwarp();
         const int nrow = __shfl_sync(FULL, pe, lane | 3) - __shfl_sync(FULL, p, lane & ~3);
-        bool ok = live && nrow <= kStRowMax;  // the same for the quad, as every break below
-        int u = 0;
-        if (ok) {
-            bool bad = false;
-            auto block_col = [&](int e) -> int {
-                const int col = staged ? sc[e - E0] : __ldg(ja + e);
-                if (col < 0 || col >= n) bad = true;
-                return col >> 2;
-            };
-            auto put = [&](int e, unsigned v) {
-                if (staged) ss[e - E0] = (unsigned char)v;
-                else slotb[e] = (unsigned char)v;
-            };
-            int t = p + 1;  // the rest of the row
-            int hc = p < pe ? block_col(p) : NONE, tc = t < pe ? block_col(t) : NONE;
-            ok = !__any_sync(gmask, bad);
-            while (ok) {
-                int mn = min(hc, tc);
-                mn = min(mn, __shfl_xor_sync(gmask, mn, 1));
-                mn = min(mn, __shfl_xor_sync(gmask, mn, 2));
-                if (mn == NONE) break;
-                if (u == 32) {  // a 33rd block column: slot bytes hold 0..31
-                    ok = false;
-                    break;
-                }
-                const unsigned hit = __ballot_sync(gmask, hc == mn || tc == mn);
+        bool ok = live && nrow <= kStRowMax;  // the same for the quad
+        bool bad = false;
+        auto block_col = [&](int e) -> int {
+            const int col = staged ? sc[e - E0] : __ldg(ja + e);
+            if (col < 0 || col >= n) bad = true;
+            return col >> 2;
+        };
+        auto put = [&](int e, unsigned v) {
+            if (staged) ss[e - E0] = (unsigned char)v;
+            else slotb[e] = (unsigned char)v;
+        };
+        int u = 0, t = p + 1;  // block columns so far, the rest of the row
+        int hc = ok && p < pe ? block_col(p) : NONE, tc = ok && t < pe ? block_col(t) : NONE;
+        ok = __any_sync(gmask, bad) ? false : ok;
+        // the warp's quads step together (each on its own takes their shuffles
+        // one quad after the other)
+        while (true) {
+            int mn = ok ? min(hc, tc) : NONE;
+            mn = min(mn, __shfl_xor_sync(FULL, mn, 1));
+            mn = min(mn, __shfl_xor_sync(FULL, mn, 2));
+            if (mn != NONE && u == 32) {  // a 33rd block column: slot bytes hold 0..31
+                ok = false;
+                mn = NONE;
+            }
+            const bool act = mn != NONE;  // the same for the quad
+            if (!__any_sync(FULL, act)) break;
+            const unsigned hit = __ballot_sync(FULL, act && (hc == mn || tc == mn)) & gmask;
+            if (act) {
                 unsigned lead = lane == __ffs(hit) - 1 ? 0x80u : 0u;
                 if (hc == mn) {
                     put(p, u | lead);
@@ -259,8 +264,8 @@ csr2bsr_count_quad_kernel(int m, int n, const int *__restrict__ ia, const int *_
                 }
                 ++u;
             }
-            if (__any_sync(gmask, bad)) ok = false;
         }
+        if (__any_sync(gmask, bad)) ok = false;
         __syncwarp();
         if (staged)
             for (int e = E0 + lane; e < E1; e += 32) slotb[e] = ss[e - E0];
@@ -575,6 +580,9 @@ csr2bsr_fill_sorted_kernel(int m, const int *__restrict__ ia, const int *__restr
     for (int wg = blockIdx.x * kFsWarps + warp; wg < nwg; wg += gridDim.x * kFsWarps) {
         const int b0 = 8 * wg;
         const int E0 = __ldg(ia + 4 * b0), E1 = __ldg(ia + min(4 * (b0 + 8), m));
+        const int b = b0 + (lane >> 2);
+        const bool mine = b < brow && !slowf[b];  // the same for the 4 lanes of a group
+        if (!__any_sync(FULL, mine)) continue;    // eight rows left to the other kernels: nothing to stage
         const bool staged = E1 - E0 <= cap;  // warp-uniform
         if (staged) {
 #pragma unroll 4
@@ -596,8 +604,7 @@ csr2bsr_fill_sorted_kernel(int m, const int *__restrict__ ia, const int *__restr
                 v = __ldg(a + p);
             }
         };
-        const int b = b0 + (lane >> 2);
-        if (b < brow && !slowf[b]) {  // the same for the 4 lanes of a group
+        if (mine) {
             const int base = bptr[b], u = bptr[b + 1] - base;
             const int r = 4 * b + q;
             int p = 0, pe = 0;
