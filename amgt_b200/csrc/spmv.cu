@@ -47,7 +47,9 @@ __device__ __forceinline__ typename ValTraits<PREC>::acc_t block_row_dot(const v
 // aligned x the blocks before it take 16-byte x loads (none do otherwise).
 // 27-point 95 x 97 x 93: fp32 67.0 -> 62.1 us, fp16 60.2 -> 53.6; 7-point 127 x
 // 129 x 127: fp32 86.2 -> 77.5, fp64 (bound by its values) 117.4 -> 117.1.  (A
-// test per block instead serialised the loads: fp64 157 us.)
+// test per block instead serialised the loads: fp64 157 us.)  Eight groups (32
+// lanes a row) take a step together or not at all, which keeps their loads
+// together: restriction of 129 x 127 x 125 (30 blocks a row) RTEXT.
 __device__ __forceinline__ int whole_end(const double *x, int k, int end)
 {
     return (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? end - 1 : k;
@@ -63,12 +65,25 @@ __device__ __forceinline__ typename ValTraits<PREC>::acc_t row_dot(const void *_
                                                                    const double *__restrict__ x, int n, int k,
                                                                    int end, int q, typename ValTraits<PREC>::acc_t acc)
 {
-    if constexpr (SAFE)
+    if constexpr (SAFE && G == 8) {
+        // the eight groups take a step together or not at all, which keeps
+        // their loads together, and the kernels keep to 32 registers
+        // (restriction of 129 x 127 x 125, 30 blocks a row, fp64: 38.5 us without
+        // this loop, 42.8 with a test of its own per group, 37.9 so)
+        const int last = 7 - (int)((threadIdx.x >> 2) & 7);  // blocks from this group's to the last group's
+#pragma unroll 1
+        for (; k + G + last < whole_end(x, k, end); k += 2 * G) {
+            const int c0 = __ldcs(idx + k), c1 = __ldcs(idx + k + G);
+            acc = block_row_dot<PREC, false>(val, x, n, k, q, c0, acc);
+            acc = block_row_dot<PREC, false>(val, x, n, k + G, q, c1, acc);
+        }
+    } else if constexpr (SAFE) {
         for (; k + G < whole_end(x, k, end); k += 2 * G) {
             const int c0 = __ldcs(idx + k), c1 = __ldcs(idx + k + G);
             acc = block_row_dot<PREC, false>(val, x, n, k, q, c0, acc);
             acc = block_row_dot<PREC, false>(val, x, n, k + G, q, c1, acc);
         }
+    }
     for (; k + G < end; k += 2 * G) {
         const int c0 = __ldcs(idx + k), c1 = __ldcs(idx + k + G);
         acc = block_row_dot<PREC, SAFE>(val, x, n, k, q, c0, acc);
@@ -142,7 +157,7 @@ __device__ __forceinline__ typename ValTraits<PREC>::acc_t row_sum(const void *_
 }
 
 template <int PREC, int LPR, bool SAFE, int V = 1>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, SAFE && LPR == 32 ? 8 : 0)
 spmv_kernel(int m, int n, int brow, const int *__restrict__ ptr, const int *__restrict__ idx,
             const void *__restrict__ val, double alpha, const double *__restrict__ x, double beta,
             double *__restrict__ y)
@@ -281,7 +296,7 @@ struct EpiArgs {
 };
 
 template <int PREC, int LPR, bool SAFE, int EPI, int V = 1>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, SAFE && LPR == 32 ? 8 : 0)
 spmv_epi_kernel(int m, int n, int brow, const int *__restrict__ ptr, const int *__restrict__ idx,
                 const void *__restrict__ val, const double *__restrict__ x, EpiArgs e)
 {
