@@ -1334,9 +1334,10 @@ __device__ __forceinline__ NumRow num_row(int b, int brA, const int *__restrict_
 // block (an FMA per entry, k ascending: the staged kernel's chain without its
 // zero terms, which change no finite sum), reading B rows straight from L1 /
 // L2; accumulators for up to kNumWideCap C blocks in shared memory, 128 bytes
-// each.  When B holds an infinity or NaN (*nonfinite), the zero terms count:
-// 0 * Inf is NaN in the staged and the gathered kernel, so every entry of A's
-// blocks is taken then, stored or not.  The row's headers are read ahead of their use.
+// each.  When B holds an infinity or NaN (*nonfinite), the zero terms count: 0
+// * Inf is NaN in the staged and the gathered kernel, so every entry of A's
+// blocks is taken then, stored or not.  The row's headers are read ahead of
+// their use.
 // 27-point 72 x 64 x 80 squared (5.5e7 pairs, 75 C blocks a row): 2.35 ms
 // against the staged kernel's 4.21 ms with 64 accumulators (longer rows in
 // global memory) and 3.48 ms with 80.  On short B rows the quads idle and the

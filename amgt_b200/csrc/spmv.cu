@@ -47,9 +47,7 @@ __device__ __forceinline__ typename ValTraits<PREC>::acc_t block_row_dot(const v
 // aligned x the blocks before it take 16-byte x loads (none do otherwise).
 // 27-point 95 x 97 x 93: fp32 67.0 -> 62.1 us, fp16 60.2 -> 53.6; 7-point 127 x
 // 129 x 127: fp32 86.2 -> 77.5, fp64 (bound by its values) 117.4 -> 117.1.  (A
-// test per block instead serialised the loads: fp64 157 us.)  Eight groups (32
-// lanes a row) take a step together or not at all, which keeps their loads
-// together: restriction of 129 x 127 x 125 (30 blocks a row) RTEXT.
+// test per block instead serialised the loads: fp64 157 us.)
 __device__ __forceinline__ int whole_end(const double *x, int k, int end)
 {
     return (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? end - 1 : k;
@@ -157,7 +155,7 @@ __device__ __forceinline__ typename ValTraits<PREC>::acc_t row_sum(const void *_
 }
 
 template <int PREC, int LPR, bool SAFE, int V = 1>
-__global__ void __launch_bounds__(256, SAFE && LPR == 32 ? 8 : 0)
+__global__ void __launch_bounds__(256, SAFE && LPR == 32 ? 8 : 0)  // (at 34 registers: 42.8 -> 52.8 us, see row_dot)
 spmv_kernel(int m, int n, int brow, const int *__restrict__ ptr, const int *__restrict__ idx,
             const void *__restrict__ val, double alpha, const double *__restrict__ x, double beta,
             double *__restrict__ y)
