@@ -471,10 +471,16 @@ int sell_fill(const std::vector<SellJob> &jobs, const int64_t *meas_host, cudaSt
         const long long steps = meas_host[kSellMeas * j], longest = meas_host[kSellMeas * j + 2];
         S.idx32 = meas_host[kSellMeas * j + 1] > 0xFFFF;
         S.holes = meas_host[kSellMeas * j + 3] != 0;
-        // long rows among short ones: the padding would outweigh the dense
-        // blocks' zeros (and 32 steps is the unit of 32-bit offsets), or one
-        // warp would walk a slice for longer than the bytes saved win
-        if (32LL * steps > 2LL * jobs[j].A->csr_nnz + 65536 || steps > 0x3FFFFFFF ||
+        // blocks of many entries: the copy, 2 or 4 bytes an entry for its column,
+        // would be no smaller than the blocks (7-point 80^3 nodes of full 4x4
+        // blocks: 105 us a product against 90 at fp64, 81 against 52 at fp16; of 4
+        // entries 44 against 91 and 29 against 53); long rows among short ones:
+        // the padding would outweigh the blocks' zeros (and 32 steps is the unit
+        // of 32-bit offsets), or one warp would walk a slice for longer than the
+        // bytes saved win
+        const int narrow = (jobs[j].storages & 12u) ? 2 : (jobs[j].storages & 2u) ? 4 : 8;  // the narrowest storage read
+        if (32LL * steps * ((S.idx32 ? 4 : 2) + narrow) >= (16LL * narrow + 6) * jobs[j].A->blc_num ||
+            32LL * steps > 2LL * jobs[j].A->csr_nnz + 65536 || steps > 0x3FFFFFFF ||
             slice_too_long(jobs[j], steps, longest, sm_count)) {
             sell_free(S, s);
             continue;

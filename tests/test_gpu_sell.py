@@ -104,23 +104,37 @@ def _coupled(orc, dims, rows, reach, count, seed=9):
     return orc.CSR(n, n, S.indptr.astype(np.int32), S.indices.astype(np.int32), S.data)
 
 
-@pytest.mark.parametrize("kind", ["padding", "one_slice"])
+@pytest.mark.parametrize("kind", ["padding", "one_slice", "full_blocks"])
 def test_operators_that_get_no_copy(amgt, orc, kind):
     """One row of 60 entries in every slice (padded to seven times the
-    entries), or one slice of 1,000 steps in an operator of 75 MB: no slice
-    columns are allocated for level 0, and the solve converges as the block
-    path does (fp64 residual)."""
+    entries), one slice of 1,000 steps in an operator of 75 MB, or full 4x4
+    blocks (4 unknowns a node): no slice columns are allocated for level 0,
+    and the solve converges as the block path does (fp64 residual)."""
+    import scipy.sparse as sp
+
     from amgt_b200.amg import AmgSolver, default_params
 
-    dims = (61, 53, 47) if kind == "padding" else (128, 128, 64)
+    dims = {"padding": (61, 53, 47), "one_slice": (128, 128, 64), "full_blocks": (30, 29, 28)}[kind]
     n = int(np.prod(dims))
-    rows = np.arange(5, n, 32) if kind == "padding" else np.array([n // 2])
-    A = _coupled(orc, dims, rows, 3000, 60 if kind == "padding" else 1000)
     Ps = orc.geometric_hierarchy(*dims)
+    if kind == "full_blocks":
+        def kron(M, B):
+            K = sp.kron(M.to_scipy(), B).tocsr()
+            K.sort_indices()
+            return orc.CSR(K.shape[0], K.shape[1], K.indptr.astype(np.int32), K.indices.astype(np.int32), K.data)
+
+        A = kron(orc.laplacian(*dims), np.eye(4) + 0.1)
+        Ps = [kron(P, np.eye(4)) for P in Ps]
+    else:
+        rows = np.arange(5, n, 32) if kind == "padding" else np.array([n // 2])
+        A = _coupled(orc, dims, rows, 3000, 60 if kind == "padding" else 1000)
+    assert orc.csr2bsr(A).nblk >= 65536
     b = A.to_scipy() @ orc.rand_uniform(6, A.n)
     steps = sliced_steps(A)
     assert (32 * steps > 2 * A.ja.size + 65536) == (kind == "padding")
     for M, copied in ((A, False), (orc.laplacian(*dims), True)):
+        if copied and kind == "full_blocks":
+            break
         amgt.set_level_policy([0])
         try:
             with AllocLog(amgt) as log:
